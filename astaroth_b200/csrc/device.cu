@@ -60,11 +60,14 @@ struct StepGraph {
     double extra; // a launch parameter the graph was captured with (CFL: time scale)
     unsigned long long launches;
     bool ghost[2]; // ghost_ok of both blocks after a replay
-    bool lo[2];    // lo_stale of both blocks after a replay
+    unsigned char lo[2]; // lo_stale of both blocks after a replay
     bool diag;     // the captured step's last substep folds the step diagnostics
 };
 
 enum { STEP_FIXED = 0, STEP_CFL = 1 };
+
+// kinds of whole-box ghost fill (0: none owed)
+enum { FILL_PERIODIC = 1, FILL_SYMMETRIC = 2, FILL_ANTISYMMETRIC = 3 };
 
 struct device_s {
     int id;
@@ -81,10 +84,11 @@ struct device_s {
     // interior (set by a full-box fill of all fields; cleared by any write to
     // the block). A fill of a block whose ghosts are already valid is skipped.
     bool ghost_ok[2];
-    // lo_stale[b] (mixed build): the last whole-box fill of block b wrote the
-    // hi parts of its ghosts only (the stencils never read the lo parts); the
-    // lo parts are filled before anything reads or partly overwrites them
-    bool lo_stale[2];
+    // lo_stale[b] (mixed build): the last whole-box fill of block b, of this
+    // kind, wrote the hi parts of its ghosts only (the stencils never read the
+    // lo parts); the lo parts are filled before anything reads or partly
+    // overwrites them
+    unsigned char lo_stale[2];
 
     CUtensorMap tmap[2];
     CentreMaps cmap[2]; // by parity of `in`: centre boxes over out hi, in lo, out lo
@@ -530,28 +534,49 @@ launch_solve(const Device d, cudaStream_t st, int step, int3 s, int3 e,
         d->diag.epoch   = d->write_epoch;
     }
     d->ghost_ok[d->cur ^ 1] = false; // the out block's ghosts are stale now
-    d->lo_stale[d->cur ^ 1] = false; // (all of them, hi and lo alike)
+    d->lo_stale[d->cur ^ 1] = 0; // (all of them, hi and lo alike)
     return AC_SUCCESS;
 }
 
-// Fills the lo parts of block b's ghosts with their periodic images if the last
-// whole-box fill of b left them (see lo_stale): the lo block has the layout of
-// the hi block with ACB_LO_NARR arrays of 8-byte elements (four bfloat16 lo
-// parts each), filled like the hi parts.
+// One whole-box ghost fill of the given kind over a block of narr arrays of
+// 8-byte elements (the fields, or the mixed build's lo block).
+static AcResult
+launch_fill(const Device d, cudaStream_t st, void* block, int narr, int kind)
+{
+    const Layout& L       = d->L;
+    const long long units = halo_units(L, narr);
+    const int blocks =
+        (int)std::max(1LL, std::min((units + 255) / 256, (long long)d->num_sms * 32));
+    const unsigned ua = (unsigned)halo_units_a(L, narr);
+    if (kind == FILL_PERIODIC)
+        halo_full_kernel<false><<<blocks, 256, 0, st>>>(L, block, ua, (unsigned)units, narr, 0);
+    else {
+        // the sign bit of every value of an element: four bf16 lo parts, two
+        // floats, or one double
+        const bool is_lo = block == (void*)d->lo[0] || block == (void*)d->lo[1];
+        const helem_t signs = is_lo        ? 0x8000800080008000ull
+                              : ACB_PAIRED ? 0x8000000080000000ull
+                                           : 0x8000000000000000ull;
+        halo_full_kernel<true><<<blocks, 256, 0, st>>>(L, block, ua, (unsigned)units, narr,
+                                                       kind == FILL_ANTISYMMETRIC ? signs : 0);
+    }
+    ACB_CUDA_CHECK(cudaGetLastError());
+    d->launches++;
+    return AC_SUCCESS;
+}
+
+// Fills the lo parts of block b's ghosts if the last whole-box fill of b left
+// them (see lo_stale): the lo block has the layout of the hi block with
+// ACB_LO_NARR arrays of 8-byte elements (four bfloat16 lo parts each), filled
+// like the hi parts.
 static AcResult
 ensure_lo_ghosts(const Device d, cudaStream_t st, int b)
 {
     if (!d->lo[b] || !d->lo_stale[b])
         return AC_SUCCESS;
-    const Layout& L       = d->L;
-    const long long units = halo_units(L, ACB_LO_NARR);
-    const int blocks =
-        (int)std::max(1LL, std::min((units + 255) / 256, (long long)d->num_sms * 32));
-    halo_full_kernel<<<blocks, 256, 0, st>>>(L, d->lo[b], (unsigned)halo_units_a(L, ACB_LO_NARR),
-                                             (unsigned)units, ACB_LO_NARR);
-    ACB_CUDA_CHECK(cudaGetLastError());
-    d->launches++;
-    d->lo_stale[b] = false;
+    if (launch_fill(d, st, d->lo[b], ACB_LO_NARR, d->lo_stale[b]) != AC_SUCCESS)
+        return AC_FAILURE;
+    d->lo_stale[b] = 0;
     return AC_SUCCESS;
 }
 
@@ -572,15 +597,10 @@ launch_halo(const Device d, cudaStream_t st, int3 s, int3 e, int f0, int f1)
     const bool whole = f0 == 0 && f1 == NUM_VTXBUF_HANDLES && s.x == 0 && s.y == 0 && s.z == 0 &&
                        e.x == L.mx && e.y == L.my && e.z == L.mz;
     if (whole) {
-        const long long units = halo_units(L);
-        const long long want  = (units + 255) / 256;
-        const int blocks = (int)std::max(1LL, std::min(want, (long long)d->num_sms * 32));
-        halo_full_kernel<<<blocks, 256, 0, st>>>(L, d->blk[d->cur], (unsigned)halo_units_a(L),
-                                                 (unsigned)units, ACB_NARR);
-        ACB_CUDA_CHECK(cudaGetLastError());
-        d->launches++;
+        if (launch_fill(d, st, d->blk[d->cur], ACB_NARR, FILL_PERIODIC) != AC_SUCCESS)
+            return AC_FAILURE;
         d->ghost_ok[d->cur] = true;
-        d->lo_stale[d->cur] = d->lo[d->cur] != nullptr;
+        d->lo_stale[d->cur] = d->lo[d->cur] ? FILL_PERIODIC : 0;
         return AC_SUCCESS;
     }
     if (ensure_lo_ghosts(d, st, d->cur) != AC_SUCCESS)
@@ -1707,6 +1727,26 @@ AcResult
 acDeviceGeneralBoundconds(const Device device, const Stream stream, const int3 start,
                           const int3 end, const AcMeshInfo config, const int3 bindex)
 {
+    const Layout& L = device->L;
+    const int bc    = config.int_params[AC_bc_type_top_x];
+    // the whole box of all fields in one launch; anything else, and what is
+    // refused, field by field
+    if (start.x <= 0 && start.y <= 0 && start.z <= 0 && end.x >= L.mx && end.y >= L.my &&
+        end.z >= L.mz) {
+        if (bc == AC_BOUNDCOND_PERIODIC)
+            return acDevicePeriodicBoundconds(device, stream, start, end);
+        if ((bc == AC_BOUNDCOND_SYMMETRIC || bc == AC_BOUNDCOND_ANTISYMMETRIC) &&
+            L.nx > NGHOST && L.ny > NGHOST && L.nz > NGHOST) {
+            cudaSetDevice(device->id);
+            const int kind = bc == AC_BOUNDCOND_SYMMETRIC ? FILL_SYMMETRIC : FILL_ANTISYMMETRIC;
+            if (launch_fill(device, stream_of(device, stream), device->blk[device->cur], ACB_NARR,
+                            kind) != AC_SUCCESS)
+                return AC_FAILURE;
+            device->ghost_ok[device->cur] = false; // no longer the periodic images
+            device->lo_stale[device->cur] = device->lo[device->cur] ? kind : 0;
+            return AC_SUCCESS;
+        }
+    }
     for (int i = 0; i < NUM_VTXBUF_HANDLES; ++i)
         if (acDeviceGeneralBoundcondStep(device, stream, (VertexBufferHandle)i, start, end, config,
                                          bindex) != AC_SUCCESS)

@@ -352,10 +352,10 @@ acNodeGeneralBoundcondStep(const Node node, const Stream stream,
 AcResult
 acNodeGeneralBoundconds(const Node node, const Stream stream, const AcMeshInfo config)
 {
-    for (int i = 0; i < NUM_VTXBUF_HANDLES; ++i)
-        if (acNodeGeneralBoundcondStep(node, stream, (VertexBufferHandle)i, config) != AC_SUCCESS)
-            return AC_FAILURE;
-    return AC_SUCCESS;
+    acNodeSynchronizeStream(node, stream);
+    const int3 z      = make_int3(0, 0, 0);
+    const int3 bindex = make_int3(-1, -1, -1);
+    return acDeviceGeneralBoundconds(node->device, stream, z, node->grid.m, config, bindex);
 }
 
 AcResult
