@@ -488,12 +488,9 @@ acEnsembleLoadMember(Ensemble e, const int member, const AcMesh host_mesh)
         return AC_FAILURE;
     }
     e->ghost_ok[e->cur] = false;
-    for (int f = 0; f < NUM_VTXBUF_HANDLES; ++f) {
-        lo16_t* lo = lo_field(mb.lo[e->cur], mb.L, f);
-        if (copy_field_range(e->stream, mb.L, mb.blk[e->cur] + fidx(mb.L, f, 0), 0,
-                             host_mesh.vertex_buffer[f], n, true, lo, &e->stage) != AC_SUCCESS)
-            return AC_FAILURE;
-    }
+    if (copy_mesh_range(e->stream, mb.L, mb.blk[e->cur], mb.lo[e->cur], 0,
+                        host_mesh.vertex_buffer, n, true, &e->stage) != AC_SUCCESS)
+        return AC_FAILURE;
     ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     return AC_SUCCESS;
 }
@@ -510,11 +507,9 @@ acEnsembleStoreMember(Ensemble e, const int member, AcMesh* host_mesh)
         fprintf(stderr, "astaroth_b200: acEnsembleStoreMember: mesh size mismatch\n");
         return AC_FAILURE;
     }
-    for (int f = 0; f < NUM_VTXBUF_HANDLES; ++f)
-        if (copy_field_range(e->stream, mb.L, mb.blk[e->cur] + fidx(mb.L, f, 0), 0,
-                             host_mesh->vertex_buffer[f], n, false, nullptr, &e->stage) !=
-            AC_SUCCESS)
-            return AC_FAILURE;
+    if (copy_mesh_range(e->stream, mb.L, mb.blk[e->cur], nullptr, 0, host_mesh->vertex_buffer, n,
+                        false, &e->stage) != AC_SUCCESS)
+        return AC_FAILURE;
     ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     return AC_SUCCESS;
 }

@@ -138,10 +138,17 @@ AcResult stage_create(StageBuf* stage, size_t max_elems);
 void stage_destroy(StageBuf* stage);
 
 // copies a flat range of a field (field: its base, block + fidx(L, f, 0))
-// between host memory (reference order) and the padded device layout through
-// the staging buffer; zeroes the lo parts of loaded values when given.
+// between the caller's memory (reference order) and the padded device layout,
+// through the staging buffer unless it is this GPU's memory; zeroes the lo parts of loaded values when given.
 AcResult copy_field_range(cudaStream_t st, const Layout& L, state_t* field, size_t s,
                           AcReal* host, size_t count, bool h2d, lo16_t* lo_field,
                           StageBuf* stage);
+
+// the same range of all eight fields (mesh: eight flat arrays, from the range's
+// first value on) between a caller's mesh and a block; in one kernel when the
+// arrays lie in this GPU's memory, else field by field. lo: the block's lo
+// parts, zeroed by a load (null where there are none).
+AcResult copy_mesh_range(cudaStream_t st, const Layout& L, state_t* block, lo16_t* lo, size_t s,
+                         AcReal* const* mesh, size_t count, bool h2d, StageBuf* stage);
 
 } // namespace acb_host

@@ -1,4 +1,6 @@
-"""The whole-box wall fill at the sizes where it can go wrong."""
+"""The whole-box wall fill and the direct copies of a mesh that lies in GPU
+memory, at the sizes where each can go wrong."""
+import ctypes as C
 import math
 
 import numpy as np
@@ -42,3 +44,57 @@ def test_whole_box_walls_equal_field_by_field(flavour, bc, n):
             got.append([dev.store_double(w) for w in range(8)])
     for w in range(8):
         assert np.array_equal(got[0][w], got[1][w]), w
+
+
+@pytest.mark.parametrize("n,start,count", [((5, 4, 3), 0, None), ((37, 29, 23), 1234, 5 * 43 + 17),
+                                           ((64, 12, 7), 0, None)])
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_mesh_in_gpu_memory_copies_like_a_host_mesh(flavour, n, start, count):
+    """Load and store of a whole mesh, or of a flat range that starts and ends
+    within a row, from and to arrays in GPU memory."""
+    import torch
+
+    prec = abi.PRECISIONS[flavour]
+    info = mesh_info(prec, n)
+    shape = tuple(m + 6 for m in n[::-1])
+    total = math.prod(shape)
+    count = total if count is None else count
+    rng = np.random.default_rng(7)
+    fields = [rng.standard_normal(shape).astype(prec.np_dtype) for _ in range(8)]
+    on_gpu = [torch.from_numpy(f).cuda() for f in fields]
+    back = [torch.full_like(t, 7.0) for t in on_gpu]
+
+    def mesh(tensors):
+        m = abi.mesh_type(prec)()
+        m.info = info
+        for w, t in enumerate(tensors):
+            m.vertex_buffer[w] = C.cast(C.c_void_p(t.data_ptr()), C.POINTER(prec.real))
+        return m
+
+    mx, my = shape[2], shape[1]
+    at = abi.int3(start % mx, start // mx % my, start // (mx * my))
+    torch.cuda.synchronize()
+    with Device(flavour, info) as dev:
+        lib = dev.lib
+        assert lib.acDeviceLoadMeshWithOffset(dev.handle, 0, mesh(on_gpu), at, at, count) == 0
+        dst = mesh(back)
+        assert lib.acDeviceStoreMeshWithOffset(dev.handle, 0, at, at, count, C.byref(dst)) == 0
+        dev.synchronize()
+        host = abi.HostMesh(prec, info)
+        dev.store_mesh(host)
+        # one field on its own
+        alone = [torch.full_like(t, 7.0) for t in on_gpu]
+        torch.cuda.synchronize()
+        dst = mesh(alone)
+        assert lib.acDeviceStoreVertexBufferWithOffset(dev.handle, 0, 5, at, at, count,
+                                                       C.byref(dst)) == 0
+        dev.synchronize()
+    for w in range(8):
+        want = np.full(total, 7.0, prec.np_dtype)
+        want[start:start + count] = fields[w].reshape(-1)[start:start + count]
+        assert np.array_equal(back[w].cpu().numpy().reshape(-1), want), w
+        want = np.zeros(total, prec.np_dtype)
+        want[start:start + count] = fields[w].reshape(-1)[start:start + count]
+        assert np.array_equal(host.fields[w].reshape(-1), want), w
+    assert np.array_equal(alone[5].cpu().numpy(), back[5].cpu().numpy())
+    assert all(bool((alone[w] == 7.0).all()) for w in range(8) if w != 5)
