@@ -33,19 +33,11 @@ using namespace acb_host;
 const SolveConfig*
 acb_host::solve_configs(int* n)
 {
-#if AC_DOUBLE_PRECISION == 1
     static const SolveConfig table[] = {
         make_solve_config<SolveCfg0, false>(),
         make_solve_config<SolveCfg1, false>(),
         make_solve_config<SolveCfg2, false>(),
     };
-#else
-    static const SolveConfig table[] = {
-        make_solve_config<SolveCfg0, false>(),
-        make_solve_config<SolveCfg1, false>(),
-        make_solve_config<SolveCfg2, false>(),
-    };
-#endif
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;
 }
@@ -333,52 +325,36 @@ acb_host::make_params(const AcMeshInfo& uniforms, const Layout& L, int step, int
     SolveParams<AcReal> P;
     memset(&P, 0, sizeof(P));
     const double inv[3] = {rp[AC_inv_dsx], rp[AC_inv_dsy], rp[AC_inv_dsz]};
-    const double c1[3]  = {3.0 / 4.0, -3.0 / 20.0, 1.0 / 60.0};
-    const double c2[4]  = {-49.0 / 18.0, 3.0 / 2.0, -3.0 / 20.0, 1.0 / 90.0};
-    const double cx[3]  = {270.0 / 720.0, -27.0 / 720.0, 2.0 / 720.0};
-    for (int a = 0; a < 3; ++a) {
-        for (int k = 0; k < 3; ++k)
-            P.c1[a][k] = (AcReal)(c1[k] * inv[a]);
-        for (int k = 0; k < 4; ++k)
-            P.c2[a][k] = (AcReal)(c2[k] * inv[a] * inv[a]);
-    }
-    const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2}; // xy, xz, yz
-    for (int p = 0; p < 3; ++p)
-        for (int k = 0; k < 3; ++k)
-            P.cx[p][k] = (AcReal)(cx[k] * inv[pa[p]] * inv[pb[p]]);
-    if (sizeof(AcReal) == 4) {
-        // the same coefficients as (c, c) lane pairs for the packed stencil sums
-        auto dup = [](AcReal c) {
-            uint32_t b;
-            memcpy(&b, &c, 4);
-            return ((unsigned long long)b << 32) | b;
-        };
-        for (int a = 0; a < 3; ++a) {
-            for (int k = 0; k < 3; ++k)
-                P.c1p[a][k] = dup(P.c1[a][k]);
-            for (int k = 0; k < 4; ++k)
-                P.c2p[a][k] = dup(P.c2[a][k]);
-        }
-        for (int r = 0; r < 3; ++r)
-            for (int k = 0; k < 3; ++k)
-                P.cxp[r][k] = dup(P.cx[r][k]);
-    }
-
+    RhsParams<AcReal>& R = P.rhs;
     const double gamma = rp[AC_gamma], cp = rp[AC_cp_sound], mu0 = rp[AC_mu0];
-    P.nu           = rp[AC_nu_visc];
-    P.eta          = rp[AC_eta];
-    P.inv_mu0      = (AcReal)(1.0 / mu0);
-    P.eta_mu0      = (AcReal)((double)rp[AC_eta] * mu0);
-    P.zeta         = rp[AC_zeta];
-    P.cs2_sound    = rp[AC_cs2_sound];
-    P.inv_cp       = (AcReal)(1.0 / cp);
-    P.gamma        = (AcReal)gamma;
-    P.gm1          = (AcReal)(gamma - 1.0);
-    P.gamma_inv_cp = (AcReal)(gamma / cp);
-    P.lnrho0       = rp[AC_lnrho0];
-    P.lnT0         = rp[AC_lnT0];
-    P.exp_lnT0     = (AcReal)exp((double)rp[AC_lnT0]);
-    P.k_heat       = (AcReal)0.001; // AC_THERMAL_CONDUCTIVITY of the module
+    const double nu = rp[AC_nu_visc], eta = rp[AC_eta], zeta = rp[AC_zeta];
+    const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2}; // xy, xz, yz
+    for (int a = 0; a < 3; ++a) {
+        const double s2 = 3.0 / 2.0 * inv[a] * inv[a];
+        const double cx = 3.0 / 8.0 * inv[pa[a]] * inv[pb[a]];
+        R.s1[a]         = (AcReal)(3.0 / 4.0 * inv[a]);
+        R.s2[a]         = (AcReal)s2;
+        R.perp_u[a]     = (AcReal)(s2 * nu);
+        R.own_u[a]      = (AcReal)(s2 * (4.0 / 3.0 * nu + zeta));
+        R.eta_a[a]      = (AcReal)(s2 * eta);
+        R.cond_s[a]     = (AcReal)(s2 * (gamma / cp));
+        R.cond_l[a]     = (AcReal)(s2 * (gamma - 1.0));
+        R.cross_u[a]    = (AcReal)(cx * (nu / 3.0 + zeta));
+        R.cross_a[a]    = (AcReal)cx;
+    }
+    R.nu          = rp[AC_nu_visc];
+    R.two_nu      = (AcReal)(2.0 * nu);
+    R.zeta        = rp[AC_zeta];
+    R.inv_mu0     = (AcReal)(1.0 / mu0);
+    R.k_ohm       = (AcReal)(eta * mu0 / (mu0 * mu0));
+    R.gamma_cp    = (AcReal)(gamma / cp);
+    R.inv_cp      = (AcReal)(1.0 / cp);
+    R.gamma       = (AcReal)gamma;
+    R.gm1         = (AcReal)(gamma - 1.0);
+    R.lnrho0      = rp[AC_lnrho0];
+    R.cs2_sound   = rp[AC_cs2_sound];
+    R.exp_lnT0    = (AcReal)exp((double)rp[AC_lnT0]);
+    R.k_heat      = (AcReal)0.001; // AC_THERMAL_CONDUCTIVITY of the module
 
     // Williamson (1980) 2N coefficients, "previous state" form
     const double alpha[3] = {0.0, -5.0 / 9.0, -153.0 / 128.0};

@@ -31,19 +31,11 @@ using namespace acb_host;
 const SolveConfig*
 acb_host::ensemble_configs(int* n)
 {
-#if AC_DOUBLE_PRECISION == 1
     static const SolveConfig table[] = {
         make_solve_config<SolveCfg0, true>(),
         make_solve_config<SolveCfg1, true>(),
         make_solve_config<SolveCfg2, true>(),
     };
-#else
-    static const SolveConfig table[] = {
-        make_solve_config<SolveCfg0, true>(),
-        make_solve_config<SolveCfg1, true>(),
-        make_solve_config<SolveCfg2, true>(),
-    };
-#endif
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;
 }
@@ -107,7 +99,7 @@ struct ensemble_s {
 
     bool desc_valid;
     std::vector<MemberDesc<AcReal>> h_desc[2];
-    std::vector<MemberParams<AcReal>> h_mp; // by task-list position (both parities)
+    std::vector<RhsParams<AcReal>> h_mp; // by task-list position (both parities)
     // launch arguments of one group of members (about 20 KB, kept off the
     // stack; the launch copies them)
     std::unique_ptr<EnsSolveArgs<AcReal>> args;
@@ -127,40 +119,6 @@ struct ensemble_s {
 };
 
 namespace {
-
-// The parts of a member's kernel parameters that its stencils and right-hand
-// sides read (MemberParams), from its full parameter set.
-MemberParams<AcReal>
-member_params(const SolveParams<AcReal>& P)
-{
-    MemberParams<AcReal> m;
-    memset(&m, 0, sizeof(m));
-#if AC_DOUBLE_PRECISION == 1
-    memcpy(m.c1, P.c1, sizeof(m.c1));
-    memcpy(m.c2, P.c2, sizeof(m.c2));
-    memcpy(m.cx, P.cx, sizeof(m.cx));
-#else
-    memcpy(m.c1p, P.c1p, sizeof(m.c1p));
-    memcpy(m.c2p, P.c2p, sizeof(m.c2p));
-    memcpy(m.cxp, P.cxp, sizeof(m.cxp));
-#endif
-    m.nu           = P.nu;
-    m.eta          = P.eta;
-    m.inv_mu0      = P.inv_mu0;
-    m.eta_mu0      = P.eta_mu0;
-    m.zeta         = P.zeta;
-    m.cs2_sound    = P.cs2_sound;
-    m.inv_cp       = P.inv_cp;
-    m.gamma        = P.gamma;
-    m.gm1          = P.gm1;
-    m.gamma_inv_cp = P.gamma_inv_cp;
-    m.lnrho0       = P.lnrho0;
-    m.lnT0         = P.lnT0;
-    m.exp_lnT0     = P.exp_lnT0;
-    m.k_heat       = P.k_heat;
-    return m;
-}
-
 
 void
 drop_graphs(Ensemble e)
@@ -188,7 +146,7 @@ build_tables(Ensemble e)
     ACB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg.kern[1], cfg.threads,
                                                                  cfg.smem));
     per_sm = std::max(per_sm, 1);
-    e->h_mp.assign(n, MemberParams<AcReal>());
+    e->h_mp.assign(n, RhsParams<AcReal>());
     for (int p = 0; p < 2; ++p) {
         std::vector<MemberDesc<AcReal>>& D = e->h_desc[p];
         D.assign(n, MemberDesc<AcReal>());
@@ -235,7 +193,7 @@ build_tables(Ensemble e)
             d.in_lo       = mb.lo[p];
             d.out_lo      = mb.lo[p ^ 1];
             if (p == 0)
-                e->h_mp[pos] = member_params(make_params(mb.uniforms, L, 0, 0));
+                e->h_mp[pos] = make_params(mb.uniforms, L, 0, 0).rhs;
             H[pos].L          = L;
             H[pos].block      = mb.blk[p];
             H[pos].unit_begin = units;

@@ -4,15 +4,19 @@
 // flat <-> padded copies.
 #pragma once
 #include <stdio.h>
+
 #include "astaroth.h"
 #include "common.cuh"
 #include "solve.cuh"
 
 // Solve tile shapes (tile width, tile height, ring depth, CTAs per SM hint)
 #if AC_DOUBLE_PRECISION == 1
-using SolveCfg0 = TileCfg<32, 4, 8, 1>;
-using SolveCfg1 = TileCfg<16, 8, 8, 1>;
-using SolveCfg2 = TileCfg<32, 2, 10, 2>;
+// 8 consumer warps of 232 registers, which hold the z queues: of a 6-plane ring
+// only four planes are in use at a time, and a tile this wide fits (with no
+// queues and the 8-plane ring that they then need, 32 x 4 tiles were the best)
+using SolveCfg0 = TileCfg<32, 8, 6, 1>;
+using SolveCfg1 = TileCfg<32, 6, 7, 1>;
+using SolveCfg2 = TileCfg<32, 4, 8, 1>;
 #elif ACB_MIXED
 // all three stage the centre values of substeps 1 and 2 by TMA; the first (the
 // default, 12 consumer warps) is the fastest on the 512^3 workload

@@ -26,18 +26,17 @@
 //     same stencils, (lnrho, ss), (ux, ax), (uy, ay), (uz, az), so a stencil
 //     point of a pair is one 8-byte shared load and its arithmetic runs in
 //     packed f32x2 lanes;
-//   - one consumer thread per (x, y) column; in single precision each thread
-//     keeps a register queue along z (its column's values of the three planes
-//     below, and running sums of the lower halves of the xz / yz diagonals),
-//     so the ring is read for the centre plane and the three above it only
-//     (112 8-byte shared loads per vertex instead of 296 values) and a plane's
-//     slot is released as soon as its own outputs are done; double precision
-//     reads all seven planes from the ring; the centre-only values (previous
-//     state, lo parts) arrive by TMA in a ring of output-plane slots (mixed
-//     substeps 1 and 2) or by plain loads (a plane ahead in double precision);
-//   - derivative coefficients arrive pre-scaled by 1/ds (and 1/ds^2) so each
-//     pencil costs 6-7 FP ops; only the 21 first, 24 second and 12 cross
-//     derivatives the right-hand sides use are formed;
+//   - one consumer thread per (x, y) column, which keeps register queues along
+//     z (values of its column, and running sums of the lower halves of the xz /
+//     yz diagonals), so the ring is read for the centre plane and the three
+//     above it only (100 8-byte shared loads per vertex in single precision, two
+//     fields each, 224 in double precision instead of 296) and a plane's slot
+//     is released as soon as its own outputs are done; the centre-only values
+//     (previous state, lo parts) arrive by TMA in a ring of output-plane slots
+//     (the mixed build) or by plain loads of what was prefetched into L1;
+//   - the stencils' coefficients are the same constants on every axis, the
+//     leading one (with 1/ds or 1/ds^2) scaling their results; only the 21
+//     first, 24 second and 12 cross derivatives the right-hand sides use count;
 //   - the mixed build keeps the state as an unevaluated sum hi + lo of a float
 //     and a bfloat16 (stored as such, widened to float in registers): stencils
 //     read hi, the update is a compensated two-sum.
@@ -47,17 +46,32 @@
 #include "common.cuh"
 #include "tma.cuh"
 
+// What the stencils' results are scaled by and the right-hand sides read: a
+// mesh's own in SolveParams, an ensemble member's in the launch's parameters (the
+// constant bank in both, where a scalar operation takes them as operands). The
+// stencils themselves, their leading coefficients taken out, need no parameter
+// (StencilCoefs).
+template <typename T>
+struct RhsParams {
+    T s1[3];                  // first derivative: axis; 3/4 / ds
+    T s2[3];                  // second derivative: axis; 3/2 / ds^2
+    T perp_u[3], own_u[3];    // s2 times nu (across the component's axis), and times
+                              // 4/3 nu + zeta (along it)
+    T eta_a[3];               // s2 times eta
+    T cond_s[3], cond_l[3];   // s2 times gamma / cp, and times gamma - 1
+    T cross_u[3], cross_a[3]; // cross derivative {xy, xz, yz}: 3/8 / (ds ds), times
+                              // nu / 3 + zeta, and as it is
+    T nu, two_nu, zeta;
+    T inv_mu0;
+    T k_ohm;    // eta mu0 / mu0^2, of |mu0 j|^2
+    T gamma_cp; // gamma / cp
+    T inv_cp, gamma, gm1, lnrho0, cs2_sound, k_heat;
+    T exp_lnT0; // exp(lnT0): T = exp(lnT0 + E) = exp_lnT0 * exp(E)
+};
+
 template <typename T>
 struct SolveParams {
-    T c1[3][3];   // first derivative: axis, k-1; pre-scaled by 1/ds
-    T c2[3][4];   // second derivative: axis, {centre, k=1..3}; pre-scaled by 1/ds^2
-    T cx[3][3];   // diagonal cross derivative: pair {xy, xz, yz}, k-1; pre-scaled
-    // single precision: c1, c2 and cx as (c, c) pairs of FP32 lanes, the
-    // coefficient operands of packed sums over the two fields of a pair
-    unsigned long long c1p[3][3], c2p[3][4], cxp[3][3];
-    T nu, eta, inv_mu0, eta_mu0, zeta;
-    T cs2_sound, inv_cp, gamma, gm1, gamma_inv_cp, lnrho0, lnT0, k_heat;
-    T exp_lnT0; // exp(lnT0): T = exp(lnT0 + E) = exp_lnT0 * exp(E)
+    RhsParams<T> rhs;
     T rkA, rkB; // out = cur + rkA * (cur - prev) + rkB * rate; rkA unused at s = 0
     // helical forcing, applied after the update at s = 2 when `forcing` != 0
     int forcing;
@@ -86,7 +100,7 @@ struct SolveGeom {
 // One member of an ensemble (many independent meshes advanced by one launch):
 // the TMA map of its `in` block, its geometry and task range and its buffers.
 // Kept in global memory, one table per buffer parity; its parameters travel
-// with the launch (MemberParams below).
+// with the launch (EnsSolveArgs::mp).
 template <typename T>
 struct __align__(128) MemberDesc {
     CUtensorMap tmap;
@@ -117,24 +131,6 @@ struct SolveArgs {
     long long total_tasks;
 };
 
-// Parameters of one ensemble member as the stencils and right-hand sides read
-// them, carried in the launch's parameter space (the constant bank, as a single
-// mesh's SolveParams are) instead of being read from memory at every use.
-template <typename T>
-struct MemberParams;
-template <>
-struct MemberParams<float> {
-    unsigned long long c1p[3][3], c2p[3][4], cxp[3][3]; // (c, c) coefficient pairs
-    float nu, eta, inv_mu0, eta_mu0, zeta;
-    float cs2_sound, inv_cp, gamma, gm1, gamma_inv_cp, lnrho0, lnT0, k_heat, exp_lnT0;
-};
-template <>
-struct MemberParams<double> {
-    double c1[3][3], c2[3][4], cx[3][3];
-    double nu, eta, inv_mu0, eta_mu0, zeta;
-    double cs2_sound, inv_cp, gamma, gm1, gamma_inv_cp, lnrho0, lnT0, k_heat, exp_lnT0;
-};
-
 // Members per ensemble launch (a launch's parameters stay within 32 KB; a
 // larger ensemble takes one launch per group of members).
 constexpr int ACB_ENS_GROUP = 64;
@@ -143,7 +139,7 @@ template <typename T>
 struct EnsSolveArgs : SolveArgs<T> {
     long long task_base;                 // first task of the group (tasks of all groups
                                          // are numbered as one list, member-major)
-    MemberParams<T> mp[ACB_ENS_GROUP];   // by position in the group
+    RhsParams<T> mp[ACB_ENS_GROUP];      // by position in the group
 };
 
 // Centre-only arrays of a substep that the ring does not carry: the previous
@@ -177,13 +173,12 @@ struct TileCfg {
     static constexpr int BX = TX_ + 8, BY = TY_ + 6;
     static constexpr int CONSUMERS = TX_ * TY_;        // one thread per (x, y) column
     static constexpr int CWARPS    = CONSUMERS / 32;   // consumer warps
-    // Single precision with 8 or 12 consumer warps: the producer is a whole
-    // warpgroup (4 warps, one of them working) that hands its registers to the
-    // consumers (setmaxnreg), so each consumer thread gets the registers its z
+    // With 8 or 12 consumer warps the producer is a whole warpgroup (4 warps,
+    // one of them working) that hands its registers to the consumers (setmaxnreg), so each consumer thread gets the registers its z
     // queues need. An SM sub-partition's 16K registers hold 2 consumer warps
     // and 1 producer warp (2 * 232 + 40 = 504 <= 512 registers a lane), or 3
     // and 1 (3 * 160 + 32 = 512): more warps to hide latency, fewer registers.
-    static constexpr bool WGSPEC = sizeof(state_t) == 4 && (CWARPS == 8 || CWARPS == 12);
+    static constexpr bool WGSPEC = CWARPS == 8 || CWARPS == 12;
     static constexpr int THREADS = CONSUMERS + (WGSPEC ? 128 : 32); // plus the producer
     static constexpr int REG_CONSUMER = CWARPS == 12 ? 160 : 232;
     static constexpr int REG_PRODUCER = CWARPS == 12 ? 32 : 40;
@@ -200,11 +195,9 @@ struct TileCfg {
     }
     static constexpr size_t smem_bytes() { return ring_bytes() + NC * centre_slot_bytes(); }
     // A task starts once the first 2 NGHOST planes are in the ring (the queue
-    // priming and the first output plane's upper half), and without queues an
-    // output plane needs all 2 NGHOST + 1 of its planes at once: a shallower
-    // ring could never hold them.
-    static_assert(NP >= (sizeof(state_t) == 4 ? 2 * NGHOST : 2 * NGHOST + 1),
-                  "ring too shallow for the planes a task waits for");
+    // priming and the first output plane's upper half): a shallower ring could
+    // never hold them.
+    static_assert(NP >= 2 * NGHOST, "ring too shallow for the planes a task waits for");
     static_assert(smem_bytes() <= 227 * 1024, "shared memory of one CTA exceeded");
 };
 
@@ -224,9 +217,8 @@ rexp<float>(float x)
 }
 
 // 1 / x: correctly rounded in double precision; in single precision the fast
-// division (within 2 ulp of the IEEE quotient for the arguments here, 1/rho and
-// 1/(rho T) of order one), 4 % of a step cheaper than the correctly rounded
-// reciprocal, whose special-case path it avoids
+// division (within 2 ulp of the IEEE quotient for the arguments here, T of order
+// one), which avoids the special-case path of the correctly rounded reciprocal
 template <typename T>
 __device__ __forceinline__ T
 rrcp(T x)
@@ -240,106 +232,15 @@ rrcp<float>(float x)
     return __fdividef(1.0f, x);
 }
 
-// first and second derivative from the six neighbours of a pencil
-template <typename T>
-__device__ __forceinline__ void
-d12(T f0, T m1, T p1, T m2, T p2, T m3, T p3, const T* c1, const T* c2, T& d1, T& d2)
-{
-    d1 = c1[0] * (p1 - m1) + c1[1] * (p2 - m2) + c1[2] * (p3 - m3);
-    d2 = c2[0] * f0 + c2[1] * (p1 + m1) + c2[2] * (p2 + m2) + c2[3] * (p3 + m3);
-}
-
-template <typename T>
-__device__ __forceinline__ T
-dd2(T f0, T m1, T p1, T m2, T p2, T m3, T p3, const T* c2)
-{
-    return c2[0] * f0 + c2[1] * (p1 + m1) + c2[2] * (p2 + m2) + c2[3] * (p3 + m3);
-}
-
-// all derivatives of one field at the thread's vertex, read from the ring
-template <typename T>
-struct FieldDerivs {
-    T v;          // value
-    T gx, gy, gz; // first derivatives
-    T xx, yy, zz; // pure second derivatives
-    T xy, xz, yz; // cross derivatives (only those requested are formed)
-};
-
-// c: pointer to the field's centre element in the centre slot;
-// zo[0..6]: element offsets of the slots of planes z-3 .. z+3 from the centre slot.
-template <typename T, int BX, bool GX, bool GY, bool GZ, bool XY, bool XZ, bool YZ, class PT>
-__device__ __forceinline__ FieldDerivs<T>
-field_derivs(const state_t* __restrict__ c, const int* zo, const PT& P)
-{
-    FieldDerivs<T> r;
-    const T f0 = (T)c[0];
-    r.v        = f0;
-    // x pencil
-    {
-        const T m1 = c[-1], p1 = c[1], m2 = c[-2], p2 = c[2], m3 = c[-3], p3 = c[3];
-        if (GX)
-            d12(f0, m1, p1, m2, p2, m3, p3, P.c1[0], P.c2[0], r.gx, r.xx);
-        else
-            r.xx = dd2(f0, m1, p1, m2, p2, m3, p3, P.c2[0]);
-    }
-    // y pencil
-    {
-        const T m1 = c[-BX], p1 = c[BX], m2 = c[-2 * BX], p2 = c[2 * BX], m3 = c[-3 * BX],
-                p3 = c[3 * BX];
-        if (GY)
-            d12(f0, m1, p1, m2, p2, m3, p3, P.c1[1], P.c2[1], r.gy, r.yy);
-        else
-            r.yy = dd2(f0, m1, p1, m2, p2, m3, p3, P.c2[1]);
-    }
-    // z pencil
-    {
-        const T m1 = c[zo[2]], p1 = c[zo[4]], m2 = c[zo[1]], p2 = c[zo[5]], m3 = c[zo[0]],
-                p3 = c[zo[6]];
-        if (GZ)
-            d12(f0, m1, p1, m2, p2, m3, p3, P.c1[2], P.c2[2], r.gz, r.zz);
-        else
-            r.zz = dd2(f0, m1, p1, m2, p2, m3, p3, P.c2[2]);
-    }
-    // diagonal cross derivatives: sum_k e_k (f(+k,+k) + f(-k,-k) - f(+k,-k) - f(-k,+k))
-    if (XY) {
-        T s = 0;
-#pragma unroll
-        for (int k = 1; k <= 3; ++k) {
-            const T a = (T)c[k + k * BX] + (T)c[-k - k * BX];
-            const T b = (T)c[k - k * BX] + (T)c[-k + k * BX];
-            s += P.cx[0][k - 1] * (a - b);
-        }
-        r.xy = s;
-    }
-    if (XZ) {
-        T s = 0;
-#pragma unroll
-        for (int k = 1; k <= 3; ++k) {
-            const T a = (T)c[zo[3 + k] + k] + (T)c[zo[3 - k] - k];
-            const T b = (T)c[zo[3 - k] + k] + (T)c[zo[3 + k] - k];
-            s += P.cx[1][k - 1] * (a - b);
-        }
-        r.xz = s;
-    }
-    if (YZ) {
-        T s = 0;
-#pragma unroll
-        for (int k = 1; k <= 3; ++k) {
-            const T a = (T)c[zo[3 + k] + k * BX] + (T)c[zo[3 - k] - k * BX];
-            const T b = (T)c[zo[3 - k] + k * BX] + (T)c[zo[3 + k] - k * BX];
-            s += P.cx[2][k - 1] * (a - b);
-        }
-        r.yz = s;
-    }
-    return r;
-}
-
-// ---- pairs of fields in packed FP32 lanes ----------------------------------
-// add/sub/mul/fma.rn.f32x2 operate on two independent FP32 lanes with the
-// rounding of the scalar operations, so a pair of fields whose stencils have
-// the same shape forms its sums and differences in half the instructions, bit
-// for bit as one field at a time. In the single-precision layout a pair is one
-// array of 8-byte (A, B) elements, so an F2 is also one 8-byte load.
+// ---- stencil values --------------------------------------------------------
+// The stencils are written once over a value type V: a double (one field), or
+// F2, the two fields of a pair array in packed FP32 lanes. add/sub/mul/
+// fma.rn.f32x2 operate on two independent FP32 lanes with the rounding of the
+// scalar operations, so a pair of fields whose stencils have the same shape
+// forms its sums and differences in half the instructions; in the layout a pair
+// is one array of 8-byte (A, B) elements, so an F2 is also one 8-byte load. The
+// rounding sequence is fixed: no operation is left for the compiler to contract,
+// so every kernel that uses a function below gets the same bits from it.
 struct F2 {
     unsigned long long v;
 };
@@ -390,390 +291,517 @@ fma2(F2 a, F2 b, F2 c)
     return r;
 }
 
-// Register queue of one pair array along z (2.5D streaming): the (A, B)
-// values of the thread's own column at the three planes below the current one
-// and, where the pair has an xz (yz) cross derivative, the lower half of that
-// derivative as running sums, both fields in packed lanes. The diagonal cross
-// derivative at plane z,
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) { return add2(a, b); }
+__device__ __forceinline__ F2 vsub(F2 a, F2 b) { return sub2(a, b); }
+__device__ __forceinline__ F2 vmul(F2 c, F2 b) { return mul2(c, b); }
+__device__ __forceinline__ F2 vfma(F2 c, F2 b, F2 d) { return fma2(c, b, d); }
+__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double vsub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double vmul(double c, double b) { return __dmul_rn(c, b); }
+__device__ __forceinline__ double vfma(double c, double b, double d) { return __fma_rn(c, b, d); }
+
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// the value type of a block's arrays
+typedef std::conditional<ACB_PAIRED, F2, double>::type V;
+
+// The stencils' coefficients with the leading one taken out, equal on every axis
+// (acc/stdlib/stdderiv.h:13-84: 3/4, -3/20, 1/60 of the first derivative; 3/2,
+// -3/20, 1/90 and -49/18 of the second; 3/8, -3/80, 1/360 of the cross one):
+//   first   d1 + r2 d2 + r3 d3,             r2 = -1/5,  r3 = 1/45
+//   second  s1 + q2 s2 + q3 s3 (+ q0 f0),   q2 = -1/10, q3 = 1/135, q0 = -49/27
+//   cross   e1 + q2 e2 + q3 e3
+// Held in registers for the whole launch: a packed operation takes no constant
+// operand, so each of the 45 (c, c) pairs that per-axis coefficients would need
+// costs a uniform load and two moves every plane. What depends on the axis scales
+// the results, as scalar operations with a constant operand.
+struct StencilCoefs {
+    V r2, r3, q0, q2, q3;
+    __device__ __forceinline__ StencilCoefs()
+    {
+        r2 = value(-1.0 / 5.0);
+        r3 = value(1.0 / 45.0);
+        q0 = value(-49.0 / 27.0);
+        q2 = value(-1.0 / 10.0);
+        q3 = value(1.0 / 135.0);
+    }
+    // opaque, so that it is kept and not formed again at each use
+    static __device__ __forceinline__ V
+    value(double c)
+    {
+        V r;
+#if AC_DOUBLE_PRECISION == 1
+        asm("mov.f64 %0, %1;" : "=d"(r) : "d"(c));
+#else
+        const float f = (float)c;
+        asm volatile("mov.b64 %0, {%1, %1};" : "=l"(r.v) : "f"(f));
+#endif
+        return r;
+    }
+};
+
+// d1 + c2 d2 + c3 d3, and the same added to a start value
+__device__ __forceinline__ V
+sum3(V c2, V c3, const V* d)
+{
+    return vfma(c3, d[2], vfma(c2, d[1], d[0]));
+}
+
+// One array's values at a vertex: centre, and the differences f(+k) - f(-k) and
+// sums of the six neighbours of each pencil (axis, k-1).
+//
+// Second differences of the mixed build as u + v with u = f(+k) - f0, v = f(-k)
+// - f0: for a smooth field u and v are exact in FP32 (Sterbenz), so f(+k) + f(-k)
+// - 2 f0 keeps its digits instead of cancelling terms of size |c0 f0| (about
+// 2.7 f / ds^2); mathematically the same stencil (c0 = -2 (c1 + c2 + c3)). This
+// is what brings the mixed build within 2.2e-7 of FP64. It is evaluated as S =
+// 2 (f(-k) - f0) + (f(+k) - f(-k)), one fused multiply-add on the two exact
+// differences (the first difference is formed anyway). The other builds, whose
+// error is that of their state, take the plain sums f(+k) + f(-k) and add c0 f0
+// (two operations per point pair instead of three).
+// First differences f(+k) - f(-k) directly, as the queues are primed, so
+// results do not depend on where a task's z segment starts.
+constexpr bool DIFF_FORM = ACB_MIXED != 0;
+
+// Queued values of a column, from plane z+ZQ-4 down to z-3: in double precision
+// those below the current plane; in single precision all but the one at z+3, so
+// that the 19 values on the axes through a vertex cost 13 shared loads instead of
+// 16 (256^3 FP32 substep 0: 477 us, with three queued values 502; substeps 1 and 2
+// 520 either way; four to six values in double precision: no gain).
+constexpr int ZQ = ACB_PAIRED ? 6 : 3;
+
+template <class V>
+struct Pencils {
+    V f0, d[3][3], s[3][3];
+};
+
+__device__ __forceinline__ void
+point_pair(F2 p, F2 m, F2 f0, F2& d, F2& s)
+{
+    d = sub2(p, m);
+    if constexpr (DIFF_FORM)
+        s = fma2(F2{0x4000000040000000ull}, sub2(m, f0), d); // (2, 2) * (m - f0) + d
+    else
+        s = add2(p, m);
+}
+
+__device__ __forceinline__ void
+point_pair(double p, double m, double, double& d, double& s)
+{
+    d = __dsub_rn(p, m);
+    s = __dadd_rn(p, m);
+}
+
+// c: the array's centre element in the centre slot; zo[3..6]: element offsets of
+// the slots of planes z .. z+3 from the centre slot; zq: the queued values of the
+// thread's own column (ZQ below), to which the value at z+3 is added.
+template <class V, int BX>
+__device__ __forceinline__ void
+load_pencils(const V* __restrict__ c, const int* zo, V* zq, Pencils<V>& p)
+{
+    // zq[k] is the value at plane z + ZQ - 4 - k
+    p.f0 = ZQ > 3 ? zq[ZQ > 3 ? ZQ - 4 : 0] : c[0];
+    V zp[3]; // z+1, z+2, z+3
+#pragma unroll
+    for (int k = 1; k <= 3; ++k)
+        zp[k - 1] = k <= ZQ - 4 ? zq[ZQ - 4 - k < 0 ? 0 : ZQ - 4 - k] : c[zo[3 + k]];
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+        point_pair(c[k], c[-k], p.f0, p.d[0][k - 1], p.s[0][k - 1]);
+        point_pair(c[k * BX], c[-k * BX], p.f0, p.d[1][k - 1], p.s[1][k - 1]);
+    }
+#pragma unroll
+    for (int k = 1; k <= 3; ++k)
+        point_pair(zp[k - 1], zq[ZQ - 4 + k], p.f0, p.d[2][k - 1], p.s[2][k - 1]);
+#pragma unroll
+    for (int k = ZQ - 1; k > 0; --k)
+        zq[k] = zq[k - 1];
+    zq[0] = ZQ > 3 ? zp[ZQ > 3 ? ZQ - 4 : 0] : p.f0;
+}
+
+// Second derivative along one axis, over its leading coefficient.
+__device__ __forceinline__ V
+second(const StencilCoefs& K, const Pencils<V>& p, int axis)
+{
+    const V* s = p.s[axis];
+    if constexpr (DIFF_FORM)
+        return sum3(K.q2, K.q3, s);
+    else
+        return vfma(K.q3, s[2], vfma(K.q2, s[1], vfma(K.q0, p.f0, s[0])));
+}
+
+// The lower halves of the xz and yz diagonal cross derivatives stream along z.
+// The derivative at plane z, over its leading coefficient,
 //   sum_k e_k (f(+k,+k) + f(-k,-k) - f(+k,-k) - f(-k,+k))
 //     = U(z) - L(z),  U(z) = sum_k e_k d_k(z+k),  L(z) = sum_k e_k d_k(z-k),
-// with d_k(w) = f(+k) - f(-k) the x (y) difference at plane w: the differences
-// of the current plane are formed for the first derivative anyway, and each
-// contributes e_k d_k(z) to L(z+k). So the queue keeps
+// with d_k(w) = f(+k) - f(-k) the x (y) difference at plane w and e = 1, q2, q3:
+// the differences of the current plane are formed for the first derivative
+// anyway, and each contributes e_k d_k(z) to L(z+k). So a queue keeps
 //   a1 = L(z),  a2 = the part of L(z+1) known so far,  a3 = that of L(z+2),
-// and advancing a plane is three fused multiply-adds (no register moves):
-//   a1 <- e1 d1(z) + a2,  a2 <- e2 d2(z) + a3,  a3 <- e3 d3(z).
+// and advancing a plane is three operations (no register moves):
+//   a1 <- a2 + d1(z),  a2 <- a3 + e2 d2(z),  a3 <- e3 d3(z).
 // Only the upper half U is read from the ring.
-struct PairQ {
-    F2 v1, v2, v3;    // (A, B) at z-1, z-2, z-3
-    F2 xa1, xa2, xa3; // xz lower half: L(z), partial L(z+1), partial L(z+2)
-    F2 ya1, ya2, ya3; // the same for yz
+struct LowerSums {
+    V a1, a2, a3;
 };
 
-// Advances the lower-half sums of one z diagonal past the plane whose
-// differences are d1, d2, d3 (e: the diagonal's (c, c) coefficient pairs).
-// The rounding sequence is fixed, so prime_pair below reproduces the sums a
-// streaming task would have built, bit for bit.
+// Advances the sums past the plane with differences d.
 __device__ __forceinline__ void
-zacc_push(F2& a1, F2& a2, F2& a3, const unsigned long long* e, F2 d1, F2 d2, F2 d3)
+push_lower(LowerSums& n, const StencilCoefs& K, const V* d)
 {
-    a1 = fma2(F2{e[0]}, d1, a2);
-    a2 = fma2(F2{e[1]}, d2, a3);
-    a3 = mul2(F2{e[2]}, d3);
+    n.a1 = vadd(n.a2, d[0]);
+    n.a2 = vfma(K.q2, d[1], n.a3);
+    n.a3 = vmul(K.q3, d[2]);
 }
 
-// Upper half U of one z diagonal (u1..u3: d_k at plane z+k).
-__device__ __forceinline__ F2
-zacc_upper(const unsigned long long* e, F2 u1, F2 u2, F2 u3)
-{
-    return fma2(F2{e[2]}, u3, fma2(F2{e[1]}, u2, mul2(F2{e[0]}, u1)));
-}
-
-// Lower-half sums of a z diagonal at the first plane of a task from the three
-// planes below it (zo[0..2]); step: 1 for xz, the row pitch for yz.
+// The sums at the first plane of a task, from the three planes below it
+// (zo[0..2]) of array c's differences along a step (1: x, BX: y), in the order
+// in which a streaming task would have added them, so bit for bit the sums it
+// would hold.
 __device__ __forceinline__ void
-zacc_prime(const F2* __restrict__ c, const int* zo, int step, const unsigned long long* e, F2& a1,
-           F2& a2, F2& a3)
+prime_lower(LowerSums& n, const StencilCoefs& K, const V* __restrict__ c, const int* zo, int step)
 {
-    auto d = [&](int plane, int k) { return sub2(c[zo[plane] + k * step], c[zo[plane] - k * step]); };
-    // plane z-3: only its third difference reaches L(z)
-    const F2 t3 = mul2(F2{e[2]}, d(0, 3));
-    // plane z-2
-    const F2 b2 = fma2(F2{e[1]}, d(1, 2), t3);
-    const F2 b3 = mul2(F2{e[2]}, d(1, 3));
-    // plane z-1
-    a1 = fma2(F2{e[0]}, d(2, 1), b2);
-    a2 = fma2(F2{e[1]}, d(2, 2), b3);
-    a3 = mul2(F2{e[2]}, d(2, 3));
+    auto d = [&](int plane, int k) { return vsub(c[zo[plane] + k * step], c[zo[plane] - k * step]); };
+    n.a1 = vadd(vfma(K.q2, d(1, 2), vmul(K.q3, d(0, 3))), d(2, 1));
+    n.a2 = vfma(K.q2, d(2, 2), vmul(K.q3, d(1, 3)));
+    n.a3 = vmul(K.q3, d(2, 3));
 }
 
-// Fills the queue of one pair array c from the ring at the first plane of a
-// task (zo[0..2]: the three planes below it).
-template <int BX, bool XZ, bool YZ, class PT>
-__device__ __forceinline__ void
-prime_pair(const F2* __restrict__ c, const int* zo, const PT& P, PairQ& Q)
+// The z diagonal cross derivative of array c along a step, and its queue advanced
+// past the plane (d: the plane's differences along the step).
+__device__ __forceinline__ V
+z_diagonal(const V* __restrict__ c, const int* zo, int step, const StencilCoefs& K, LowerSums& n,
+           const V* d)
 {
-    Q.v1 = c[zo[2]];
-    Q.v2 = c[zo[1]];
-    Q.v3 = c[zo[0]];
-    if (XZ)
-        zacc_prime(c, zo, 1, P.cxp[1], Q.xa1, Q.xa2, Q.xa3);
-    if (YZ)
-        zacc_prime(c, zo, BX, P.cxp[2], Q.ya1, Q.ya2, Q.ya3);
+    V u[3];
+#pragma unroll
+    for (int k = 1; k <= 3; ++k)
+        u[k - 1] = vsub(c[zo[3 + k] + k * step], c[zo[3 + k] - k * step]);
+    u[0]      = vsub(u[0], n.a1);
+    const V x = sum3(K.q2, K.q3, u);
+    push_lower(n, K, d);
+    return x;
 }
 
-template <bool GX_, bool GY_, bool GZ_, bool XY_, bool XZ_, bool YZ_>
-struct DFlags {
-    static constexpr bool GX = GX_, GY = GY_, GZ = GZ_, XY = XY_, XZ = XZ_, YZ = YZ_;
+// The derivatives of one array at a vertex, over their leading coefficients:
+// gradient, second derivatives by axis, and the cross derivatives that the
+// right-hand sides use of a vector's component.
+struct Derivs {
+    V g[3], d2[3], xa, xb;
 };
 
-// The z-diagonal cross derivative of kind XK (xz, else yz) of both fields of
-// a pair, in packed lanes: upper half from the ring, lower half queued.
-template <bool XK, int BX, class PT>
 __device__ __forceinline__ void
-zcross_pair(const F2* __restrict__ c, const int* zo, const PT& P, const PairQ& Q,
-            float& sA, float& sB)
+gradient_and_second(const StencilCoefs& K, const Pencils<V>& p, Derivs& r)
 {
-    constexpr int step = XK ? 1 : BX;
-    F2 u[3];
 #pragma unroll
-    for (int k = 1; k <= 3; ++k) {
-        const int z = zo[3 + k];
-        u[k - 1]    = sub2(c[z + k * step], c[z - k * step]);
+    for (int a = 0; a < 3; ++a) {
+        r.g[a]  = sum3(K.r2, K.r3, p.d[a]);
+        r.d2[a] = second(K, p, a);
     }
-    const F2 s = sub2(zacc_upper(P.cxp[XK ? 1 : 2], u[0], u[1], u[2]), XK ? Q.xa1 : Q.ya1);
-    upk2(s, sA, sB);
 }
 
-// Advances a pair's queue by one plane (after every use of it): F0 and the
-// x / y differences DX, DY of the plane just done.
-template <bool XZ, bool YZ, class PT>
+// Component I of a vector: a field, or the pair of a velocity and a vector
+// potential component. Its cross derivatives with the other axes in order (x
+// first); na, nb: the queues of its z diagonals (components 0 and 1: nb; 2: xz in
+// na, yz in nb).
+template <int I, int BX>
 __device__ __forceinline__ void
-push_queue(PairQ& Q, const PT& P, F2 F0, const F2* DX, const F2* DY)
+vector_component(const V* __restrict__ c, const int* zo, V* zq, const StencilCoefs& K,
+                 LowerSums& na, LowerSums& nb, V& f0, Derivs& r)
 {
-    if (XZ)
-        zacc_push(Q.xa1, Q.xa2, Q.xa3, P.cxp[1], DX[0], DX[1], DX[2]);
-    if (YZ)
-        zacc_push(Q.ya1, Q.ya2, Q.ya3, P.cxp[2], DY[0], DY[1], DY[2]);
-    Q.v3 = Q.v2;
-    Q.v2 = Q.v1;
-    Q.v1 = F0;
-}
-
-// The derivatives of the two fields of one pair array c at once: every pencil
-// sum and difference, the xy diagonals and the z diagonals in packed lanes
-// (each stencil point one 8-byte load); the coefficient sums. Second
-// derivatives in difference form (below). F0 returns the pair's centre values.
-template <int BX, class FA, class FB, class PT>
-__device__ __forceinline__ void
-pair_derivs_q(const F2* __restrict__ c, const int* zo, const PT& P,
-              PairQ& Q, FieldDerivs<float>& rA, FieldDerivs<float>& rB, F2& F0)
-{
-    static_assert(FA::XY == FB::XY && FA::XZ == FB::XZ && FA::YZ == FB::YZ,
-                  "the fields of a pair have the same cross derivatives");
-    F0 = c[0];
-    float a0, b0;
-    upk2(F0, a0, b0);
-    rA.v = a0;
-    rB.v = b0;
-    F2 DX[3], SX[3], DY[3], SY[3], DZ[3], SZ[3];
-    // Second differences as u + v with u = f(+k) - f0, v = f(-k) - f0: for a
-    // smooth field u and v are exact in FP32 (Sterbenz), so f(+k) + f(-k) - 2 f0
-    // keeps its digits instead of cancelling terms of size |c0 f0| (about
-    // 2.7 f / ds^2); mathematically the same stencil (c0 = -2 (c1 + c2 + c3)).
-    // The FP32 build, whose error is that of its FP32 state, keeps the plain
-    // sums f(+k) + f(-k) and adds c0 f0 (two packed operations per point pair
-    // instead of three); the difference form is what brings the mixed build
-    // within 2.2e-7 of FP64.
-    // First differences f(+k) - f(-k) directly, as prime_pair forms the queued
-    // ones, so results do not depend on where a task's z segment starts.
-    // The difference form is evaluated as S = 2 (f(-k) - f0) + (f(+k) - f(-k)),
-    // one fused multiply-add on the two exact differences (the first
-    // difference is formed anyway): a single rounding of the same value,
-    // three packed operations per point pair instead of four.
-    constexpr bool DIFF_FORM = ACB_MIXED != 0;
-    auto dsum = [&](F2 p, F2 m, F2& D, F2& S) {
-        D = sub2(p, m);
-        if constexpr (DIFF_FORM)
-            S = fma2(F2{0x4000000040000000ull}, sub2(m, F0), D); // (2, 2) * (m - f0) + D
-        else
-            S = add2(p, m);
-    };
-#pragma unroll
-    for (int k = 1; k <= 3; ++k) {
-        dsum(c[k], c[-k], DX[k - 1], SX[k - 1]);
-        dsum(c[k * BX], c[-k * BX], DY[k - 1], SY[k - 1]);
-    }
-    dsum(c[zo[4]], Q.v1, DZ[0], SZ[0]);
-    dsum(c[zo[5]], Q.v2, DZ[1], SZ[1]);
-    dsum(c[zo[6]], Q.v3, DZ[2], SZ[2]);
-    // Coefficient sums sum_k c_k d_k of both fields at once, with (c, c)
-    // coefficient pairs from the kernel parameters.
-    auto sum3 = [&](const unsigned long long* cp, const F2* d, float& oa, float& ob) {
-        F2 r = mul2(F2{cp[0]}, d[0]);
-        r    = fma2(F2{cp[1]}, d[1], r);
-        upk2(fma2(F2{cp[2]}, d[2], r), oa, ob);
-    };
-    float gA, gB;
-    if (FA::GX || FB::GX) {
-        sum3(P.c1p[0], DX, gA, gB);
-        if (FA::GX) rA.gx = gA;
-        if (FB::GX) rB.gx = gB;
-    }
-    if (FA::GY || FB::GY) {
-        sum3(P.c1p[1], DY, gA, gB);
-        if (FA::GY) rA.gy = gA;
-        if (FB::GY) rB.gy = gB;
-    }
-    if (FA::GZ || FB::GZ) {
-        sum3(P.c1p[2], DZ, gA, gB);
-        if (FA::GZ) rA.gz = gA;
-        if (FB::GZ) rB.gz = gB;
-    }
-    if constexpr (DIFF_FORM) {
-        sum3(P.c2p[0] + 1, SX, rA.xx, rB.xx);
-        sum3(P.c2p[1] + 1, SY, rA.yy, rB.yy);
-        sum3(P.c2p[2] + 1, SZ, rA.zz, rB.zz);
-    }
-    else {
-        // c0 f0 + sum_k c_k (f(+k) + f(-k))
-        auto sum4 = [&](const unsigned long long* cp, const F2* d, float& oa, float& ob) {
-            F2 r = mul2(F2{cp[0]}, F0);
-            r    = fma2(F2{cp[1]}, d[0], r);
-            r    = fma2(F2{cp[2]}, d[1], r);
-            upk2(fma2(F2{cp[3]}, d[2], r), oa, ob);
-        };
-        sum4(P.c2p[0], SX, rA.xx, rB.xx);
-        sum4(P.c2p[1], SY, rA.yy, rB.yy);
-        sum4(P.c2p[2], SZ, rA.zz, rB.zz);
-    }
-
-    // xy diagonals (the whole stencil from the centre plane)
-    if (FA::XY) {
-        F2 E[3];
+    Pencils<V> p;
+    load_pencils<V, BX>(c, zo, zq, p);
+    f0 = p.f0;
+    gradient_and_second(K, p, r);
+    if constexpr (I < 2) { // xy diagonals (the whole stencil from the centre plane)
+        V e[3];
 #pragma unroll
         for (int k = 1; k <= 3; ++k) {
             const int pp = k + k * BX, mm = -k - k * BX, pm = k - k * BX, mp = -k + k * BX;
-            E[k - 1] = sub2(add2(c[pp], c[mm]), add2(c[pm], c[mp]));
+            e[k - 1] = vsub(vadd(c[pp], c[mm]), vadd(c[pm], c[mp]));
         }
-        sum3(P.cxp[0], E, rA.xy, rB.xy);
+        r.xa = sum3(K.q2, K.q3, e);
+        r.xb = z_diagonal(c, zo, I == 0 ? 1 : BX, K, nb, p.d[I]);
     }
-
-    // z diagonals (both fields have the same kinds)
-    if (FA::XZ)
-        zcross_pair<true, BX>(c, zo, P, Q, rA.xz, rB.xz);
-    if (FA::YZ)
-        zcross_pair<false, BX>(c, zo, P, Q, rA.yz, rB.yz);
-
-    push_queue<FA::XZ, FA::YZ>(Q, P, F0, DX, DY);
+    else {
+        r.xa = z_diagonal(c, zo, 1, K, na, p.d[0]);
+        r.xb = z_diagonal(c, zo, BX, K, nb, p.d[1]);
+    }
 }
 
-// Derivative flags of the eight fields: what the right-hand sides use.
-//                   GX     GY     GZ     XY     XZ     YZ
-#define ACB_D_LNRHO true, true, true, false, false, false
-#define ACB_D_UUX true, true, true, true, true, false
-#define ACB_D_UUY true, true, true, true, false, true
-#define ACB_D_UUZ true, true, true, false, true, true
-#define ACB_D_AX false, true, true, true, true, false
-#define ACB_D_AY true, false, true, true, false, true
-#define ACB_D_AZ true, true, false, false, true, true
-#define ACB_D_SS true, true, true, false, false, false
-
-template <typename T, class PT>
-__device__ __forceinline__ void rhs_terms(const FieldDerivs<T>& lr, const FieldDerivs<T>& ux,
-                                          const FieldDerivs<T>& uy, const FieldDerivs<T>& uz,
-                                          const FieldDerivs<T>& ax, const FieldDerivs<T>& ay,
-                                          const FieldDerivs<T>& az, const FieldDerivs<T>& ss,
-                                          const PT& P, T roc[ACB_NF], T cur[ACB_NF]);
-
-// Right-hand sides of the eight fields at one vertex, every stencil operand
-// read from the ring.
-template <typename T, int BX, int FIELD, class PT>
+// A scalar (or the pair lnrho, entropy).
+template <int BX>
 __device__ __forceinline__ void
-mhd_rhs(const state_t* __restrict__ c, const int* zo, const PT& P, T roc[ACB_NF],
-        T cur[ACB_NF])
+scalar_field(const V* __restrict__ c, const int* zo, V* zq, const StencilCoefs& K, V& f0, Derivs& r)
 {
-    const auto lr = field_derivs<T, BX, ACB_D_LNRHO>(c + 0 * FIELD, zo, P);
-    const auto ux = field_derivs<T, BX, ACB_D_UUX>(c + 1 * FIELD, zo, P);
-    const auto uy = field_derivs<T, BX, ACB_D_UUY>(c + 2 * FIELD, zo, P);
-    const auto uz = field_derivs<T, BX, ACB_D_UUZ>(c + 3 * FIELD, zo, P);
-    const auto ax = field_derivs<T, BX, ACB_D_AX>(c + 4 * FIELD, zo, P);
-    const auto ay = field_derivs<T, BX, ACB_D_AY>(c + 5 * FIELD, zo, P);
-    const auto az = field_derivs<T, BX, ACB_D_AZ>(c + 6 * FIELD, zo, P);
-    const auto ss = field_derivs<T, BX, ACB_D_SS>(c + 7 * FIELD, zo, P);
-    rhs_terms(lr, ux, uy, uz, ax, ay, az, ss, P, roc, cur);
+    Pencils<V> p;
+    load_pencils<V, BX>(c, zo, zq, p);
+    f0 = p.f0;
+    gradient_and_second(K, p, r);
 }
 
-// The same with the z register queues (single-precision stencils), one pair
-// array at a time: (lnrho, ss), (ux, ax), (uy, ay), (uz, az). cur2 returns the
-// centre values of each array.
-template <int BX, int FIELD, class PT>
-__device__ __forceinline__ void
-mhd_rhs_q(const F2* __restrict__ c, const int* zo, const PT& P,
-          float roc[ACB_NF], float cur[ACB_NF], F2 cur2[ACB_NARR], PairQ (&Q)[ACB_NARR])
-{
-    FieldDerivs<float> lr, ux, uy, uz, ax, ay, az, ss;
-    pair_derivs_q<BX, DFlags<ACB_D_LNRHO>, DFlags<ACB_D_SS>>(c + 0 * FIELD, zo, P, Q[0], lr, ss,
-                                                             cur2[0]);
-    pair_derivs_q<BX, DFlags<ACB_D_UUX>, DFlags<ACB_D_AX>>(c + 1 * FIELD, zo, P, Q[1], ux, ax,
-                                                           cur2[1]);
-    pair_derivs_q<BX, DFlags<ACB_D_UUY>, DFlags<ACB_D_AY>>(c + 2 * FIELD, zo, P, Q[2], uy, ay,
-                                                           cur2[2]);
-    pair_derivs_q<BX, DFlags<ACB_D_UUZ>, DFlags<ACB_D_AZ>>(c + 3 * FIELD, zo, P, Q[3], uz, az,
-                                                           cur2[3]);
-    rhs_terms(lr, ux, uy, uz, ax, ay, az, ss, P, roc, cur);
-}
+// What the right-hand sides are made of (stencil_kernel.ac:355-528, regrouped):
+// values and gradients of lnrho and entropy, first = gamma/cp lap s + (gamma-1)
+// lap lnrho, velocity and its gradient g[i][a], the off-diagonal sums T of the
+// gradient (01, 02, 12), B, mu0 j = grad div A - lap A, the viscous terms nu lap u
+// + (nu/3 + zeta) grad div u, eta lap A.
+template <typename T>
+struct Terms {
+    T lnrho, ss, glr[3], gs[3], first;
+    T u[3], g[3][3], t01, t02, t12, b[3], j[3];
+    T visc[3], resist[3];
+};
 
-template <int BX, int FIELD, class PT>
-__device__ __forceinline__ void
-prime_queues(const F2* __restrict__ c, const int* zo, const PT& P,
-             PairQ (&Q)[ACB_NARR])
-{
-    prime_pair<BX, false, false>(c + 0 * FIELD, zo, P, Q[0]);
-    prime_pair<BX, true, false>(c + 1 * FIELD, zo, P, Q[1]);
-    prime_pair<BX, false, true>(c + 2 * FIELD, zo, P, Q[2]);
-    prime_pair<BX, true, true>(c + 3 * FIELD, zo, P, Q[3]);
-}
-
-// Right-hand sides from the derivative sets (stencil_kernel.ac:355-528,
-// restated; same terms).
+// Right-hand sides, roc in field order. With E = gamma s/cp + (gamma-1)(lnrho -
+// lnrho0), T = exp(lnT0 + E): rho enters only as 1/rho = exp(-lnrho), since the
+// heating terms that carry a factor rho are divided by rho T; and both gradients
+// in the heat conduction, gamma/cp grad s + (gamma-1) grad lnrho and gamma (grad
+// s/cp + grad lnrho) - grad lnrho, are the same vector.
 template <typename T, class PT>
 __device__ __forceinline__ void
-rhs_terms(const FieldDerivs<T>& lr, const FieldDerivs<T>& ux, const FieldDerivs<T>& uy,
-          const FieldDerivs<T>& uz, const FieldDerivs<T>& ax, const FieldDerivs<T>& ay,
-          const FieldDerivs<T>& az, const FieldDerivs<T>& ss, const PT& P,
-          T roc[ACB_NF], T cur[ACB_NF])
+rhs_from(const PT& P, const Terms<T>& m, T roc[ACB_NF])
 {
-    cur[0] = lr.v;
-
-    cur[1] = ux.v;
-    cur[2] = uy.v;
-    cur[3] = uz.v;
-    cur[4] = ax.v;
-    cur[5] = ay.v;
-    cur[6] = az.v;
-    cur[7] = ss.v;
-
-    const T u0 = ux.v, u1 = uy.v, u2 = uz.v;
-    const T divu = ux.gx + uy.gy + uz.gz;
-
-    // continuity: -u.grad(lnrho) - div(u)
-    roc[0] = -(u0 * lr.gx + u1 * lr.gy + u2 * lr.gz) - divu;
-
-    // B = curl A
-    const T B0 = az.gy - ay.gz;
-    const T B1 = ax.gz - az.gx;
-    const T B2 = ay.gx - ax.gy;
-    const T lapA0 = ax.xx + ax.yy + ax.zz;
-    const T lapA1 = ay.xx + ay.yy + ay.zz;
-    const T lapA2 = az.xx + az.yy + az.zz;
-
-    // induction: u x B + eta lap(A)
-    roc[4] = (u1 * B2 - u2 * B1) + P.eta * lapA0;
-    roc[5] = (u2 * B0 - u0 * B2) + P.eta * lapA1;
-    roc[6] = (u0 * B1 - u1 * B0) + P.eta * lapA2;
-
-    // j = (grad div A - lap A) / mu0
-    const T j0 = P.inv_mu0 * ((ax.xx + ay.xy + az.xz) - lapA0);
-    const T j1 = P.inv_mu0 * ((ax.xy + ay.yy + az.yz) - lapA1);
-    const T j2 = P.inv_mu0 * ((ax.xz + ay.yz + az.zz) - lapA2);
-
-    // traceless strain S
-    const T third = (T)1 / (T)3, twothird = (T)2 / (T)3, half = (T)0.5;
-    const T S00   = twothird * ux.gx - third * (uy.gy + uz.gz);
-    const T S11   = twothird * uy.gy - third * (ux.gx + uz.gz);
-    const T S22   = twothird * uz.gz - third * (ux.gx + uy.gy);
-    const T S01   = half * (ux.gy + uy.gx);
-    const T S02   = half * (ux.gz + uz.gx);
-    const T S12   = half * (uy.gz + uz.gy);
-
-    // thermodynamics: E = gamma s / cp + (gamma - 1)(lnrho - lnrho0)
-    const T E       = P.gamma * ss.v * P.inv_cp + P.gm1 * (lr.v - P.lnrho0);
+    const T E       = rfma(P.gamma_cp, m.ss, P.gm1 * (m.lnrho - P.lnrho0));
     const T expE    = rexp<T>(E);
     const T cs2     = P.cs2_sound * expE;
-    const T rho     = rexp<T>(lr.v);
-    const T inv_rho = rrcp<T>(rho);
+    const T inv_rho = rexp<T>(-m.lnrho);
+    const T inv_T   = rrcp<T>(P.exp_lnT0 * expE);
 
-    // momentum
-    const T gd0 = ux.xx + uy.xy + uz.xz;
-    const T gd1 = ux.xy + uy.yy + uz.yz;
-    const T gd2 = ux.xz + uy.yz + uz.zz;
-    const T jxB0 = j1 * B2 - j2 * B1;
-    const T jxB1 = j2 * B0 - j0 * B2;
-    const T jxB2 = j0 * B1 - j1 * B0;
-    const T lapu0 = ux.xx + ux.yy + ux.zz;
-    const T lapu1 = uy.xx + uy.yy + uy.zz;
-    const T lapu2 = uz.xx + uz.yy + uz.zz;
-    const T Sg0   = S00 * lr.gx + S01 * lr.gy + S02 * lr.gz;
-    const T Sg1   = S01 * lr.gx + S11 * lr.gy + S12 * lr.gz;
-    const T Sg2   = S02 * lr.gx + S12 * lr.gy + S22 * lr.gz;
-    roc[1] = -(ux.gx * u0 + ux.gy * u1 + ux.gz * u2) - cs2 * (P.inv_cp * ss.gx + lr.gx) +
-             inv_rho * jxB0 + P.nu * (lapu0 + third * gd0 + (T)2 * Sg0) + P.zeta * gd0;
-    roc[2] = -(uy.gx * u0 + uy.gy * u1 + uy.gz * u2) - cs2 * (P.inv_cp * ss.gy + lr.gy) +
-             inv_rho * jxB1 + P.nu * (lapu1 + third * gd1 + (T)2 * Sg1) + P.zeta * gd1;
-    roc[3] = -(uz.gx * u0 + uz.gy * u1 + uz.gz * u2) - cs2 * (P.inv_cp * ss.gz + lr.gz) +
-             inv_rho * jxB2 + P.nu * (lapu2 + third * gd2 + (T)2 * Sg2) + P.zeta * gd2;
+    // continuity: -u.grad(lnrho) - div(u)
+    const T divu = m.g[0][0] + m.g[1][1] + m.g[2][2];
+    roc[0] = -rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], rfma(m.u[2], m.glr[2], divu)));
 
-    // entropy
-    // T = exp(lnT0 + E) = exp(lnT0) exp(E): the exponential of E is formed
-    // above already
-    const T inv_pT = rrcp<T>(rho * (P.exp_lnT0 * expE));
-    const T SS     = S00 * S00 + S01 * S01 + S02 * S02 + S01 * S01 + S11 * S11 + S12 * S12 +
-                 S02 * S02 + S12 * S12 + S22 * S22;
-    const T heat = P.eta_mu0 * (j0 * j0 + j1 * j1 + j2 * j2) + (T)2 * rho * P.nu * SS +
-                   P.zeta * rho * divu * divu;
-    const T lap_s  = ss.xx + ss.yy + ss.zz;
-    const T lap_lr = lr.xx + lr.yy + lr.zz;
-    const T first  = P.gamma_inv_cp * lap_s + P.gm1 * lap_lr;
-    const T sec0 = P.gamma_inv_cp * ss.gx + P.gm1 * lr.gx;
-    const T sec1 = P.gamma_inv_cp * ss.gy + P.gm1 * lr.gy;
-    const T sec2 = P.gamma_inv_cp * ss.gz + P.gm1 * lr.gz;
-    const T thi0 = P.gamma * (P.inv_cp * ss.gx + lr.gx) - lr.gx;
-    const T thi1 = P.gamma * (P.inv_cp * ss.gy + lr.gy) - lr.gy;
-    const T thi2 = P.gamma * (P.inv_cp * ss.gz + lr.gz) - lr.gz;
-    // cp * chi with chi = K / (rho cp)
-    const T hc = P.k_heat * inv_rho * (first + (sec0 * thi0 + sec1 * thi1 + sec2 * thi2));
-    roc[7]     = -(u0 * ss.gx + u1 * ss.gy + u2 * ss.gz) + inv_pT * heat + hc;
+    // induction: u x B + eta lap(A)
+    roc[4] = rfma(m.u[1], m.b[2], rfma(-m.u[2], m.b[1], m.resist[0]));
+    roc[5] = rfma(m.u[2], m.b[0], rfma(-m.u[0], m.b[2], m.resist[1]));
+    roc[6] = rfma(m.u[0], m.b[1], rfma(-m.u[1], m.b[0], m.resist[2]));
+
+    // traceless strain: diagonal s, off-diagonal t / 2
+    const T third = (T)1 / (T)3;
+    const T d3    = third * divu;
+    const T s0 = m.g[0][0] - d3, s1 = m.g[1][1] - d3, s2 = m.g[2][2] - d3;
+
+    // momentum: -(u.grad)u - cs2 (grad s / cp + grad lnrho) + j x B / rho +
+    //   nu (lap u + grad div u / 3 + 2 S.grad lnrho) + zeta grad div u
+    T pr[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        pr[i] = rfma(P.inv_cp, m.gs[i], m.glr[i]);
+    const T jb0 = rfma(m.j[1], m.b[2], -(m.j[2] * m.b[1]));
+    const T jb1 = rfma(m.j[2], m.b[0], -(m.j[0] * m.b[2]));
+    const T jb2 = rfma(m.j[0], m.b[1], -(m.j[1] * m.b[0]));
+    const T sg0 = rfma(s0 + s0, m.glr[0], rfma(m.t01, m.glr[1], m.t02 * m.glr[2]));
+    const T sg1 = rfma(m.t01, m.glr[0], rfma(s1 + s1, m.glr[1], m.t12 * m.glr[2]));
+    const T sg2 = rfma(m.t02, m.glr[0], rfma(m.t12, m.glr[1], (s2 + s2) * m.glr[2]));
+    const T irm = inv_rho * P.inv_mu0;
+    auto momentum = [&](int i, T jb, T sg) {
+        T r = rfma(-m.u[0], m.g[i][0], m.visc[i]);
+        r   = rfma(-m.u[1], m.g[i][1], r);
+        r   = rfma(-m.u[2], m.g[i][2], r);
+        r   = rfma(P.nu, sg, r);
+        r   = rfma(-cs2, pr[i], r);
+        return rfma(irm, jb, r);
+    };
+    roc[1] = momentum(0, jb0, sg0);
+    roc[2] = momentum(1, jb1, sg1);
+    roc[3] = momentum(2, jb2, sg2);
+
+    // entropy: -u.grad(s) + (eta mu0 j.j + 2 rho nu S:S + zeta rho div(u)^2) / (rho T)
+    //   + K / rho (first + |gamma (grad s / cp + grad lnrho) - grad lnrho|^2)
+    const T off = rfma(m.t01, m.t01, rfma(m.t02, m.t02, m.t12 * m.t12));
+    const T ss  = rfma(s0, s0, rfma(s1, s1, rfma(s2, s2, (T)0.5 * off)));
+    const T jj  = rfma(m.j[0], m.j[0], rfma(m.j[1], m.j[1], m.j[2] * m.j[2]));
+    const T heat = rfma(P.two_nu, ss, rfma(P.zeta * divu, divu, (P.k_ohm * inv_rho) * jj));
+    T cond = m.first;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const T q = rfma(P.gamma, pr[i], -m.glr[i]);
+        cond      = rfma(q, q, cond);
+    }
+    T r    = rfma(inv_T, heat, (P.k_heat * inv_rho) * cond);
+    r      = rfma(-m.u[0], m.gs[0], r);
+    r      = rfma(-m.u[1], m.gs[1], r);
+    roc[7] = rfma(-m.u[2], m.gs[2], r);
+}
+
+// Register queues of one thread's column along z: the values of each array at
+// the planes of ZQ, and the lower sums of the z diagonals, xz of component 0, yz
+// of 1, xz and yz of 2, of (u, A), or of u and then A in double precision.
+struct ColumnQ {
+    V v[ACB_NARR][ZQ];
+    LowerSums n[ACB_PAIRED ? 4 : 8];
+};
+
+// Fills the queues from the ring at the first plane of a task (zo[0..2]: the
+// three planes below it).
+template <int BX, int FIELD>
+__device__ __forceinline__ void
+prime_queues(const V* __restrict__ c, const int* zo, const StencilCoefs& K, ColumnQ& Q)
+{
+#pragma unroll
+    for (int a = 0; a < ACB_NARR; ++a)
+#pragma unroll
+        for (int k = 0; k < ZQ; ++k)
+            Q.v[a][k] = c[a * FIELD + zo[ZQ - 1 - k]];
+#pragma unroll
+    for (int w = 0; w < (ACB_PAIRED ? 1 : 2); ++w) {
+        const V *x = c + (1 + 3 * w) * FIELD, *y = x + FIELD, *z = y + FIELD;
+        prime_lower(Q.n[4 * w + 0], K, x, zo, 1);
+        prime_lower(Q.n[4 * w + 1], K, y, zo, BX);
+        prime_lower(Q.n[4 * w + 2], K, z, zo, 1);
+        prime_lower(Q.n[4 * w + 3], K, z, zo, BX);
+    }
+}
+
+// Adds the cross derivatives of a vector's components that belong to each
+// component of its grad div (k: their coefficients).
+template <typename T>
+__device__ __forceinline__ void
+add_cross_terms(const T* k, const T (&xa)[3], const T (&xb)[3], T (&r)[3])
+{
+    r[0] = rfma(k[0], xa[1], rfma(k[1], xa[2], r[0]));
+    r[1] = rfma(k[0], xa[0], rfma(k[2], xb[2], r[1]));
+    r[2] = rfma(k[1], xb[0], rfma(k[2], xb[1], r[2]));
+}
+
+// The velocity's terms from its derivatives (g, d2: [component][axis]).
+template <typename T>
+__device__ __forceinline__ void
+velocity_terms(const RhsParams<T>& P, const T (&g)[3][3], const T (&d2)[3][3], const T (&xa)[3],
+               const T (&xb)[3], Terms<T>& m)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int a = i == 0 ? 1 : 0, b = i == 2 ? 1 : 2;
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            m.g[i][x] = P.s1[x] * g[i][x];
+        m.visc[i] = rfma(P.own_u[i], d2[i][i], rfma(P.perp_u[a], d2[i][a], P.perp_u[b] * d2[i][b]));
+    }
+    add_cross_terms(P.cross_u, xa, xb, m.visc);
+    m.t01 = m.g[0][1] + m.g[1][0];
+    m.t02 = m.g[0][2] + m.g[2][0];
+    m.t12 = m.g[1][2] + m.g[2][1];
+}
+
+// The vector potential's: B, eta lap A and mu0 j = grad div A - lap A.
+template <typename T>
+__device__ __forceinline__ void
+potential_terms(const RhsParams<T>& P, const T (&g)[3][3], const T (&d2)[3][3], const T (&xa)[3],
+                const T (&xb)[3], Terms<T>& m)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int a = i == 0 ? 1 : 0, b = i == 2 ? 1 : 2;
+        m.b[i] = i == 0 ? rfma(P.s1[1], g[2][1], -(P.s1[2] * g[1][2]))
+                        : (i == 1 ? rfma(P.s1[2], g[0][2], -(P.s1[0] * g[2][0]))
+                                  : rfma(P.s1[0], g[1][0], -(P.s1[1] * g[0][1])));
+        m.resist[i] = rfma(P.eta_a[0], d2[i][0], rfma(P.eta_a[1], d2[i][1], P.eta_a[2] * d2[i][2]));
+        m.j[i]      = rfma(-P.s2[a], d2[i][a], -(P.s2[b] * d2[i][b]));
+    }
+    add_cross_terms(P.cross_a, xa, xb, m.j);
+}
+
+// Density's and entropy's.
+template <typename T>
+__device__ __forceinline__ void
+scalar_terms(const RhsParams<T>& P, const T (&gl)[3], const T (&gs)[3], const T (&dl)[3],
+             const T (&ds)[3], Terms<T>& m)
+{
+    T f = P.cond_l[0] * dl[0];
+    f   = rfma(P.cond_l[1], dl[1], f);
+    f   = rfma(P.cond_l[2], dl[2], f);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        f        = rfma(P.cond_s[a], ds[a], f);
+        m.glr[a] = P.s1[a] * gl[a];
+        m.gs[a]  = P.s1[a] * gs[a];
+    }
+    m.first = f;
+}
+
+// Right-hand sides at one vertex and the centre values of each array; advances
+// the queues by a plane. Single precision: the stencils of two fields at once,
+// (lnrho, ss), (ux, ax), (uy, ay), (uz, az). `late` is called before the stencils
+// of density and entropy, the last.
+template <int BX, int FIELD, class F>
+__device__ __forceinline__ void
+mhd_rhs_q(const V* __restrict__ c, const int* zo, const StencilCoefs& K,
+          const RhsParams<AcReal>& P, AcReal roc[ACB_NF], V cur[ACB_NARR], ColumnQ& Q, F late)
+{
+    typedef AcReal T;
+    Terms<T> m;
+#if AC_DOUBLE_PRECISION == 0
+    T g[2][3][3], d2[2][3][3], xa[2][3], xb[2][3];
+    auto component = [&](auto I, LowerSums& na, LowerSums& nb) {
+        constexpr int i = I.value;
+        Derivs r;
+        vector_component<i, BX>(c + (1 + i) * FIELD, zo, Q.v[1 + i], K, na, nb, cur[1 + i], r);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            upk2(r.g[x], g[0][i][x], g[1][i][x]);
+            upk2(r.d2[x], d2[0][i][x], d2[1][i][x]);
+        }
+        upk2(r.xa, xa[0][i], xa[1][i]);
+        upk2(r.xb, xb[0][i], xb[1][i]);
+        T unused;
+        upk2(cur[1 + i], m.u[i], unused);
+        (void)unused;
+    };
+    component(std::integral_constant<int, 0>{}, Q.n[0], Q.n[0]);
+    component(std::integral_constant<int, 1>{}, Q.n[1], Q.n[1]);
+    component(std::integral_constant<int, 2>{}, Q.n[2], Q.n[3]);
+    potential_terms(P, g[1], d2[1], xa[1], xb[1], m);
+    velocity_terms(P, g[0], d2[0], xa[0], xb[0], m);
+    late();
+    Derivs r;
+    scalar_field<BX>(c, zo, Q.v[0], K, cur[0], r);
+    upk2(cur[0], m.lnrho, m.ss);
+    T gl[3], gs[3], dl[3], ds[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        upk2(r.g[x], gl[x], gs[x]);
+        upk2(r.d2[x], dl[x], ds[x]);
+    }
+    scalar_terms(P, gl, gs, dl, ds, m);
+#else
+    auto vector = [&](int f, LowerSums* n, auto terms) {
+        Derivs r[3];
+        vector_component<0, BX>(c + f * FIELD, zo, Q.v[f], K, n[0], n[0], cur[f], r[0]);
+        vector_component<1, BX>(c + (f + 1) * FIELD, zo, Q.v[f + 1], K, n[1], n[1], cur[f + 1], r[1]);
+        vector_component<2, BX>(c + (f + 2) * FIELD, zo, Q.v[f + 2], K, n[2], n[3], cur[f + 2], r[2]);
+        T g[3][3], d2[3][3], xa[3], xb[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                g[i][x]  = r[i].g[x];
+                d2[i][x] = r[i].d2[x];
+            }
+            xa[i] = r[i].xa;
+            xb[i] = r[i].xb;
+        }
+        terms(g, d2, xa, xb);
+    };
+    vector(4, Q.n + 4, [&](auto& g, auto& d2, auto& xa, auto& xb) {
+        potential_terms(P, g, d2, xa, xb, m);
+    });
+    vector(1, Q.n, [&](auto& g, auto& d2, auto& xa, auto& xb) {
+        velocity_terms(P, g, d2, xa, xb, m);
+    });
+    late();
+    Derivs l, e;
+    scalar_field<BX>(c, zo, Q.v[0], K, cur[0], l);
+    scalar_field<BX>(c + 7 * FIELD, zo, Q.v[7], K, cur[7], e);
+    m.u[0]  = cur[1];
+    m.u[1]  = cur[2];
+    m.u[2]  = cur[3];
+    m.lnrho = cur[0];
+    m.ss    = cur[7];
+    scalar_terms(P, l.g, e.g, l.d2, e.d2, m);
+#endif
+    rhs_from(P, m, roc);
 }
 
 // Helical forcing at interior vertex (i, j, k) (stencil_kernel.ac:611-648 with
@@ -919,6 +947,17 @@ load_centre(const Layout& L, const state_t* out, long long id, CentreVals& c)
     for (int f = 0; f < ACB_NF; ++f)
         if (STEP > 0)
             c.prev[f] = out[fidx(L, f, id)];
+}
+
+// The previous state of the vertex a plane above into L1.
+template <int STEP>
+__device__ __forceinline__ void
+prefetch_centre(const Layout& L, const state_t* out, long long id)
+{
+#pragma unroll
+    for (int f = 0; f < ACB_NF; ++f)
+        if (STEP > 0)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(out + fidx(L, f, id)));
 }
 
 // The lo parts of pair array ar from a lo element (two bf16x2 words, the
@@ -1080,20 +1119,17 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
         ok = mbar_wait_bounded(&full[(q + l) % NP], ((q + l) / NP) & 1u);
     ok = __all_sync(0xffffffffu, ok);
 
-    // single precision streams with the z register queues (2.5D) over the pair
-    // arrays; double precision has no registers to spare for them and reads
-    // every operand from the ring
-    constexpr bool QZ = ACB_PAIRED;
-    acb::PairQ Q[ACB_NARR];
-    if constexpr (QZ) {
+    acb::ColumnQ Q;
+    const acb::StencilCoefs K;
+    {
         if (ok && act) {
             const uint32_t sc = (q + NGHOST) % NP;
             int zo[7];
 #pragma unroll
             for (int dz = -NGHOST; dz <= NGHOST; ++dz)
                 zo[dz + NGHOST] = ((int)((q + NGHOST + dz) % NP) - (int)sc) * PLANE;
-            const acb::F2* c = reinterpret_cast<const acb::F2*>(ring) + (size_t)sc * PLANE + col;
-            acb::prime_queues<BX, FIELD>(c, zo, P, Q);
+            const acb::V* c = reinterpret_cast<const acb::V*>(ring) + (size_t)sc * PLANE + col;
+            acb::prime_queues<BX, FIELD>(c, zo, K, Q);
         }
         // the three planes below the first output plane now live in the queues
         __syncwarp();
@@ -1104,18 +1140,10 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
 
     // forcing (s = 2 with forcing; single precision): the column's phase factor
     float fcxy = 0.f, fsxy = 0.f, fcz = 0.f, fsz = 0.f;
-    if constexpr (STEP == 3 && QZ)
+    if constexpr (STEP == 3 && ACB_PAIRED)
         acb::forcing_column(a.P, i, j, fcxy, fsxy);
     (void)fcxy;
     (void)fsxy;
-
-    // double precision (no queues, registers to spare for it): the centre
-    // values of the next plane are loaded a plane ahead
-    constexpr bool PREF = !QZ;
-    CentreVals cv_next;
-    if constexpr (PREF)
-        if (act)
-            load_centre<STEP>(L, out, lidx(L, i, j, tg.k0), cv_next);
 
     for (int p = 0; p < tg.nout; ++p) {
         if (ok) {
@@ -1138,7 +1166,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
         }
         const int k = tg.k0 + p;
         float fcb = 0.f, fsb = 0.f; // the plane's forcing phase factor
-        if constexpr (STEP == 3 && QZ) {
+        if constexpr (STEP == 3 && ACB_PAIRED) {
             if ((p & 31) == 0) // lane l: plane p + l
                 acb::forcing_plane(a.P, k + lane, fcz, fsz);
             fcb = __shfl_sync(0xffffffffu, fcz, p & 31);
@@ -1151,27 +1179,29 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
             const uint32_t sc  = (q + p + NGHOST) % NP;
             int zo[7];
 #pragma unroll
-            for (int dz = -NGHOST; dz <= NGHOST; ++dz) {
-                if (QZ && dz < 0)
-                    continue;
+            for (int dz = 0; dz <= NGHOST; ++dz) {
                 const int sd    = (int)((q + p + NGHOST + dz) % NP);
                 zo[dz + NGHOST] = (sd - (int)sc) * PLANE;
             }
             T fo[3] = {0, 0, 0};
-            if constexpr (QZ) {
+            if constexpr (ACB_PAIRED) {
                 // previous state and lo parts of this vertex: plain loads issued
-                // first, or (CT) read from the centre slot after the right-hand
-                // sides, which keeps their registers free through the stencils
+                // first, or after the right-hand sides, which keeps their
+                // registers free through the stencils: lo parts, and (CT) what
+                // is read from the centre slot
                 CentreVals2 cv;
                 if constexpr (!CT) {
-                    load_centre2<STEP>(L, out, in_lo, out_lo, id, cv);
+                    if (!ACB_MIXED)
+                        load_centre2<STEP>(L, out, in_lo, out_lo, id, cv);
                     if (p + 1 < tg.nout)
                         prefetch_centre2<STEP>(L, out, in_lo, out_lo, id + L.plane);
                 }
                 const acb::F2* c = reinterpret_cast<const acb::F2*>(ring) + (size_t)sc * PLANE + col;
-                float roc[ACB_NF], cur[ACB_NF];
+                float roc[ACB_NF];
                 acb::F2 cur2[ACB_NARR];
-                acb::mhd_rhs_q<BX, FIELD>(c, zo, P, roc, cur, cur2, Q);
+                acb::mhd_rhs_q<BX, FIELD>(c, zo, K, P, roc, cur2, Q, [] {});
+                if constexpr (!CT && ACB_MIXED)
+                    load_centre2<STEP>(L, out, in_lo, out_lo, id, cv);
                 if constexpr (STEP == 3)
                     acb::forcing_from<T>(a.P, fcxy, fsxy, fcb, fsb, fo);
                 if constexpr (CT) {
@@ -1274,18 +1304,21 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     }
                     diag_add(dacc, v[0], v[1], v[2], v[3]);
                 }
-                (void)cur;
                 (void)dh;
                 (void)dl;
             }
             else {
-                // double precision: previous state loaded a plane ahead
-                CentreVals cv = cv_next;
                 if (p + 1 < tg.nout)
-                    load_centre<STEP>(L, out, id + L.plane, cv_next);
+                    prefetch_centre<STEP>(L, out, id + L.plane);
                 const state_t* c = reinterpret_cast<const state_t*>(ring) + (size_t)sc * PLANE + col;
                 T roc[ACB_NF], cur[ACB_NF];
-                acb::mhd_rhs<T, BX, FIELD>(c, zo, P, roc, cur);
+                // the previous state, prefetched into L1 a plane ago, is loaded
+                // before the last two fields' stencils: it arrives under them and
+                // holds its registers through the least of the work (256^3
+                // substep 1: 1083 us, loaded first 1104, after all 1175)
+                CentreVals cv;
+                acb::mhd_rhs_q<BX, FIELD>(c, zo, K, P, roc, cur, Q,
+                                          [&] { load_centre<STEP>(L, out, id, cv); });
                 if constexpr (STEP == 3)
                     acb::forcing_at<T>(a.P, i, j, k, fo);
                 T dv[4];
@@ -1311,7 +1344,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
         // with the queues the centre plane is done with; without them the
         // plane three below it
         if (lane == 0)
-            mbar_arrive(&empty[(q + p + (QZ ? NGHOST : 0)) % NP]);
+            mbar_arrive(&empty[(q + p + NGHOST) % NP]);
         if constexpr (CT) {
             if (lane == 0)
                 mbar_arrive(&empty_c[oq % Cfg::NC]);
@@ -1321,7 +1354,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
     // the planes of the task not released yet
     __syncwarp();
     if (lane == 0)
-        for (int l = tg.nout + (QZ ? NGHOST : 0); l < nload; ++l)
+        for (int l = tg.nout + NGHOST; l < nload; ++l)
             mbar_arrive(&empty[(q + l) % NP]);
     q += nload;
     return true;
@@ -1575,7 +1608,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
                                                      empty_c, oq, dacc);
         }
         else {
-            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG>(a, a.g, a.P, t, a.out, a.in_lo, a.out_lo,
+            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG>(a, a.g, a.P.rhs, t, a.out, a.in_lo, a.out_lo,
                                                     ring, full, empty, &abort_flag, q, centre,
                                                     full_c, empty_c, oq, dacc);
         }
