@@ -698,8 +698,10 @@ run_reduce(const Device d, cudaStream_t st, int rtype, int nin, const int* handl
         // sets: the request, then each input as a scalar (a scalar request's
         // own field excepted)
         const int ns = !c.wide ? 1 : (nin == RED_SCAL ? nf : 1 + nf);
-        if (ns == 1)
-            reduce3_kernel<256><<<(unsigned)blocks, 256, 0, st>>>(a);
+        if (ns == 1 && nin == RED_SCAL)
+            reduce_sets_kernel<256, RED_SCAL, 1><<<(unsigned)blocks, 256, 0, st>>>(a);
+        else if (ns == 1)
+            reduce_sets_kernel<256, RED_VEC, 1><<<(unsigned)blocks, 256, 0, st>>>(a);
         else if (nin == RED_SCAL)
             reduce_sets_kernel<256, RED_SCAL, 2><<<(unsigned)blocks, 256, 0, st>>>(a);
         else if (ns == 4)
@@ -732,7 +734,12 @@ run_reduce(const Device d, cudaStream_t st, int rtype, int nin, const int* handl
         c.n += ns;
         return AC_SUCCESS;
     }
-    reduce_kernel<256><<<(unsigned)blocks, 256, 0, st>>>(a);
+    if (nin == RED_SCAL)
+        reduce_kernel<256, RED_SCAL><<<(unsigned)blocks, 256, 0, st>>>(a);
+    else if (nin == RED_VEC)
+        reduce_kernel<256, RED_VEC><<<(unsigned)blocks, 256, 0, st>>>(a);
+    else
+        reduce_kernel<256, RED_ALFVEN><<<(unsigned)blocks, 256, 0, st>>>(a);
     ACB_CUDA_CHECK(cudaGetLastError());
     d->launches++;
     ACB_CUDA_CHECK(cudaMemcpyAsync(d->h_result, d->red_result, sizeof(double),
@@ -1124,30 +1131,11 @@ replay_steps(const Device device, cudaStream_t st, int kind, unsigned long long 
 //   uu_dt   = cdt dsmin / (|umax| + sqrt(cs2_sound))
 //   visc_dt = cdtv dsmin^2 / max(max(nu, eta), max(gamma, chi = 0))
 //   dt      = (AcReal)timescale * (AcReal)min(uu_dt, visc_dt)
-// Here the same formula runs in one GPU thread on the max |u| that
-// reduce3_kernel left in device memory, in double precision (the reference
-// host code uses long double), with umax first rounded to AcReal as the
-// reference's acReduceVec returns it. Nothing returns to the host, so a whole
-// simulation step, time step included, is one CUDA graph.
-struct CflParams {
-    double cdt, cdtv, dsmin, cs2, nu, eta, gamma;
-    AcReal timescale;
-};
-
-// rec: dt of the last step, simulated time, steps taken
-static __global__ void
-cfl_kernel(const double* umax, double* rec, const CflParams p)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
-    const double u       = (double)(AcReal)umax[0];
-    const double uu_dt   = p.cdt * p.dsmin / (fabs(u) + sqrt(p.cs2));
-    const double visc_dt = p.cdtv * p.dsmin * p.dsmin / fmax(fmax(p.nu, p.eta), fmax(p.gamma, 0.0));
-    const AcReal dt      = p.timescale * (AcReal)fmin(uu_dt, visc_dt);
-    rec[0]               = (double)dt;
-    rec[1] += (double)dt;
-    rec[2] += 1.0;
-}
+// Here the same formula (cfl_step) runs on the GPU, in the thread that completes
+// the max |u| reduction, in double precision (the reference host code uses long
+// double), with umax first rounded to AcReal as the reference's acReduceVec
+// returns it. Nothing returns to the host, so a whole simulation step, time step
+// included, is one CUDA graph.
 
 // The formula's parameters from the uniform mirror. AC_dsmin as the
 // standalone's config loader sets it (min of AC_dsx, AC_dsy, AC_dsz) where the
@@ -1179,7 +1167,7 @@ cfl_params(const Device d, AcReal timescale, CflParams& cp)
     return AC_SUCCESS;
 }
 
-// max |u| into d->red_result, the time step into d->cfl, then the three
+// max |u| into d->red_result and the time step into d->cfl, then the three
 // substeps reading it: 3 x (ghost fill, solve, swap).
 static AcResult
 enqueue_step_cfl(const Device d, cudaStream_t st, const CflParams& cp)
@@ -1189,11 +1177,11 @@ enqueue_step_cfl(const Device d, cudaStream_t st, const CflParams& cp)
     long long blocks;
     if (reduce_args(d, RTYPE_MAX, RED_VEC, hu, a, blocks) != AC_SUCCESS)
         return AC_FAILURE;
-    reduce3_kernel<256><<<(unsigned)blocks, 256, 0, st>>>(a);
+    a.cfl     = cp;
+    a.cfl_rec = d->cfl;
+    reduce_sets_kernel<256, RED_VEC, 1><<<(unsigned)blocks, 256, 0, st>>>(a);
     ACB_CUDA_CHECK(cudaGetLastError());
-    cfl_kernel<<<1, 32, 0, st>>>(d->red_result, d->cfl, cp);
-    ACB_CUDA_CHECK(cudaGetLastError());
-    d->launches += 2;
+    d->launches++;
     const int3 m0 = make_int3(0, 0, 0);
     const int3 m1 = make_int3(d->L.mx, d->L.my, d->L.mz);
     const int3 n0 = make_int3(NGHOST, NGHOST, NGHOST);

@@ -27,6 +27,25 @@ constexpr int ACB_RED_SETS = 7;
 // and a vector, with room to spare)
 constexpr int ACB_RED_RECORD = 16;
 
+// Parameters of the Courant time step, and its record: dt of the last step,
+// simulated time, steps taken.
+struct CflParams {
+    double cdt, cdtv, dsmin, cs2, nu, eta, gamma;
+    AcReal timescale;
+};
+
+__device__ __forceinline__ void
+cfl_step(double umax, const CflParams& p, double* rec)
+{
+    const double u       = (double)(AcReal)umax;
+    const double uu_dt   = p.cdt * p.dsmin / (fabs(u) + sqrt(p.cs2));
+    const double visc_dt = p.cdtv * p.dsmin * p.dsmin / fmax(fmax(p.nu, p.eta), fmax(p.gamma, 0.0));
+    const AcReal dt      = p.timescale * (AcReal)fmin(uu_dt, visc_dt);
+    rec[0]               = (double)dt;
+    rec[1] += (double)dt;
+    rec[2] += 1.0;
+}
+
 struct ReduceArgs {
     Layout L;
     const state_t* f[6];
@@ -38,6 +57,8 @@ struct ReduceArgs {
     double* partials;   // gridDim.x doubles of scratch
     unsigned* counter;  // scratch counter, zero between launches
     double* result;
+    double* cfl_rec; // not null: the last block also takes the time step that
+    CflParams cfl;   // set 0's maximum (max |u|) allows
 };
 
 __device__ __forceinline__ double
@@ -72,6 +93,29 @@ red_load(const ReduceArgs& a, int w, long long id)
     return v;
 }
 
+// Both fields of the pair array of input w, one 8-byte element: input w's own
+// value and its partner's.
+__device__ __forceinline__ void
+red_load_pair(const ReduceArgs& a, int w, long long id, double& own, double& other)
+{
+#if AC_DOUBLE_PRECISION == 0
+    // the field's base is its array's, or one value further (lane 1)
+    const unsigned lane  = (unsigned)(((uintptr_t)a.f[w] >> 2) & 1u);
+    const float2 e       = reinterpret_cast<const float2*>(a.f[w] - lane)[id];
+    own                  = (double)(lane ? e.y : e.x);
+    other                = (double)(lane ? e.x : e.y);
+#if ACB_MIXED
+    // likewise the pair's bf16x2 word of the lo element
+    const uint32_t l = *reinterpret_cast<const uint32_t*>(a.lo[w] - lane + id * ACB_LO_STEP);
+    const uint32_t x = l << 16, y = l & 0xffff0000u;
+    own += (double)__uint_as_float(lane ? y : x);
+    other += (double)__uint_as_float(lane ? x : y);
+#endif
+#else
+    own = other = red_load(a, w, id);
+#endif
+}
+
 // |v|^2 of a vector, with one fixed rounding sequence for every reduction
 // that uses it (the length for MAX / MIN, the square for RMS), so that a pass
 // computing several of them returns what separate passes return, bit for bit.
@@ -81,22 +125,22 @@ red_len2(double x, double y, double z)
     return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
 }
 
+// The filtered value of one vertex from its nin input values.
+template <int NIN>
 __device__ __forceinline__ double
-red_filter(const ReduceArgs& a, long long id)
+red_filter(int rt, const double* v)
 {
-    const int rt = a.rtype;
-    if (a.nin == RED_SCAL) {
-        const double v = red_load(a, 0, id);
+    if (NIN == RED_SCAL) {
         if (rt == RTYPE_RMS)
-            return __dmul_rn(v, v);
+            return __dmul_rn(v[0], v[0]);
         if (rt == RTYPE_RMS_EXP) {
-            const double e = exp(v);
+            const double e = exp(v[0]);
             return e * e;
         }
-        return v; // MAX, MIN, SUM
+        return v[0]; // MAX, MIN, SUM
     }
-    const double x = red_load(a, 0, id), y = red_load(a, 1, id), z = red_load(a, 2, id);
-    if (a.nin == RED_VEC) {
+    const double x = v[0], y = v[1], z = v[2];
+    if (NIN == RED_VEC) {
         if (rt == RTYPE_RMS)
             return red_len2(x, y, z);
         if (rt == RTYPE_RMS_EXP) {
@@ -106,7 +150,7 @@ red_filter(const ReduceArgs& a, long long id)
         return sqrt(red_len2(x, y, z)); // MAX, MIN, SUM of the length
     }
     // Alfven speed with density exponent d
-    const double d  = red_load(a, 3, id);
+    const double d  = v[3];
     const double b2 = x * x + y * y + z * z;
     const double q  = 4.0 * M_PI * exp(d);
     if (rt == RTYPE_ALFVEN_RMS)
@@ -114,25 +158,62 @@ red_filter(const ReduceArgs& a, long long id)
     return sqrt(b2) / sqrt(q);
 }
 
-template <int THREADS>
+// Calls f(values) for every vertex of the rows of this warp, a lane's vertices
+// in ascending order. A lane loads its next ACB_RED_AHEAD vertices' inputs
+// before it uses the first, so that a row is a few waits on memory instead of one
+// for each 32 vertices. 512^3, against one vertex at a time: |u| alone FP32 504 us
+// instead of 682, mixed 836 instead of 882, FP64 598 instead of 671; the vector with
+// all fields it reads 874, 1068 and 572 us instead of 1340, 1646 and 960; rms_exp
+// 324, 337 and 269 instead of 386, 915 and 506; a field with its partner takes 7 to
+// 14 % longer, 285 us in FP32.
+constexpr int ACB_RED_AHEAD = 4;
+
+template <int THREADS, int NF, class Load, class F>
+__device__ __forceinline__ void
+red_rows(const ReduceArgs& a, Load load, F f)
+{
+    const int lane    = threadIdx.x & 31;
+    const unsigned gw = (blockIdx.x * THREADS + threadIdx.x) >> 5;
+    const unsigned nw = (gridDim.x * THREADS) >> 5;
+    const int rx      = a.end.x - a.start.x;
+    const unsigned ry = (unsigned)(a.end.y - a.start.y);
+    for (unsigned r = gw; r < (unsigned)a.rows; r += nw) {
+        const unsigned kq    = r / ry;
+        const long long base = lidx(a.L, a.start.x, a.start.y + (int)(r - kq * ry),
+                                    a.start.z + (int)kq);
+        int i = lane;
+        for (; i + 32 * (ACB_RED_AHEAD - 1) < rx; i += 32 * ACB_RED_AHEAD) {
+            double v[ACB_RED_AHEAD][NF];
+#pragma unroll
+            for (int u = 0; u < ACB_RED_AHEAD; ++u)
+                load(base + i + 32 * u, v[u]);
+#pragma unroll
+            for (int u = 0; u < ACB_RED_AHEAD; ++u)
+                f(v[u]);
+        }
+        for (; i < rx; i += 32) {
+            double v[NF];
+            load(base + i, v);
+            f(v);
+        }
+    }
+}
+
+template <int THREADS, int NIN>
 __global__ void __launch_bounds__(THREADS)
 reduce_kernel(const ReduceArgs a)
 {
-    const Layout& L = a.L;
-    const int lane  = threadIdx.x & 31;
-    const int wid   = threadIdx.x >> 5;
-    const long long gw  = ((long long)blockIdx.x * THREADS + threadIdx.x) >> 5;
-    const long long nw  = ((long long)gridDim.x * THREADS) >> 5;
-    const int rx        = a.end.x - a.start.x;
-    const int ry        = a.end.y - a.start.y;
-    double acc          = red_identity(a.rtype);
-    for (long long r = gw; r < a.rows; r += nw) {
-        const int j          = a.start.y + (int)(r % ry);
-        const int k          = a.start.z + (int)(r / ry);
-        const long long base = lidx(L, a.start.x, j, k);
-        for (int i = lane; i < rx; i += 32)
-            acc = red_combine(a.rtype, acc, red_filter(a, base + i));
-    }
+    const int lane = threadIdx.x & 31;
+    const int wid  = threadIdx.x >> 5;
+    double acc     = red_identity(a.rtype);
+    red_rows<THREADS, NIN>(
+        a,
+        [&](long long id, double* v) {
+#pragma unroll
+            for (int w = 0; w < NIN; ++w)
+                v[w] = red_load(a, w, id);
+        },
+        [&](const double* v) { acc = red_combine(a.rtype, acc, red_filter<NIN>(a.rtype, v)); });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         acc = red_combine(a.rtype, acc, __shfl_xor_sync(0xffffffffu, acc, o));
@@ -173,131 +254,25 @@ reduce_kernel(const ReduceArgs a)
     }
 }
 
-// MAX, MIN and the RMS sum of one scalar field or one vector's length in a
-// single pass (a.rtype unused): three accumulators, each combined in exactly
-// the order reduce_kernel combines its one, so result[0..2] equal the MAX,
-// MIN and RMS passes' results bit for bit. partials holds 3 * gridDim.x.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS)
-reduce3_kernel(const ReduceArgs a)
-{
-    const Layout& L = a.L;
-    const int lane  = threadIdx.x & 31;
-    const int wid   = threadIdx.x >> 5;
-    const long long gw  = ((long long)blockIdx.x * THREADS + threadIdx.x) >> 5;
-    const long long nw  = ((long long)gridDim.x * THREADS) >> 5;
-    const int rx        = a.end.x - a.start.x;
-    const int ry        = a.end.y - a.start.y;
-    double mx = -INFINITY, mn = INFINITY, sm = 0.0;
-    for (long long r = gw; r < a.rows; r += nw) {
-        const int j          = a.start.y + (int)(r % ry);
-        const int k          = a.start.z + (int)(r / ry);
-        const long long base = lidx(L, a.start.x, j, k);
-        for (int i = lane; i < rx; i += 32) {
-            const long long id = base + i;
-            double m, q;
-            if (a.nin == RED_SCAL) {
-                m = red_load(a, 0, id);
-                q = __dmul_rn(m, m);
-            }
-            else {
-                q = red_len2(red_load(a, 0, id), red_load(a, 1, id), red_load(a, 2, id));
-                m = sqrt(q);
-            }
-            mx = fmax(mx, m);
-            mn = fmin(mn, m);
-            sm = sm + q;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        sm = sm + __shfl_xor_sync(0xffffffffu, sm, o);
-    }
-    __shared__ double wmx[THREADS / 32], wmn[THREADS / 32], wsm[THREADS / 32];
-    __shared__ bool last;
-    if (lane == 0) {
-        wmx[wid] = mx;
-        wmn[wid] = mn;
-        wsm[wid] = sm;
-    }
-    __syncthreads();
-    const unsigned G = gridDim.x;
-    if (threadIdx.x == 0) {
-        double bx = wmx[0], bn = wmn[0], bs = wsm[0];
-        for (int w = 1; w < THREADS / 32; ++w) {
-            bx = fmax(bx, wmx[w]);
-            bn = fmin(bn, wmn[w]);
-            bs = bs + wsm[w];
-        }
-        a.partials[blockIdx.x]         = bx;
-        a.partials[G + blockIdx.x]     = bn;
-        a.partials[2 * G + blockIdx.x] = bs;
-        __threadfence();
-        const unsigned done = atomicAdd(a.counter, 1u);
-        last                = (done == G - 1);
-    }
-    __syncthreads();
-    if (last) {
-        // the fixed-order fold of reduce_kernel, for each accumulator
-        __threadfence();
-        const volatile double* P = a.partials;
-        double vx = -INFINITY, vn = INFINITY, vs = 0.0;
-        for (int b = threadIdx.x; b < (int)G; b += THREADS) {
-            vx = fmax(vx, P[b]);
-            vn = fmin(vn, P[G + b]);
-            vs = vs + P[2 * G + b];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            vx = fmax(vx, __shfl_xor_sync(0xffffffffu, vx, o));
-            vn = fmin(vn, __shfl_xor_sync(0xffffffffu, vn, o));
-            vs = vs + __shfl_xor_sync(0xffffffffu, vs, o);
-        }
-        if (lane == 0) {
-            wmx[wid] = vx;
-            wmn[wid] = vn;
-            wsm[wid] = vs;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double bx = wmx[0], bn = wmn[0], bs = wsm[0];
-            for (int w = 1; w < THREADS / 32; ++w) {
-                bx = fmax(bx, wmx[w]);
-                bn = fmin(bn, wmn[w]);
-                bs = bs + wsm[w];
-            }
-            a.result[0] = bx;
-            a.result[1] = bn;
-            a.result[2] = bs;
-            *a.counter  = 0u; // ready for the next launch on this stream
-        }
-    }
-}
-
-// MAX, MIN and the RMS sum of several sets in one pass: set 0 is one scalar
-// field (NIN = RED_SCAL, input 0) or one vector's length (NIN = RED_VEC, inputs
-// 0-2); sets 1 .. NS-1 are the scalar fields of the inputs that follow
+// MAX, MIN and the RMS sum of one or several sets in one pass: set 0 is one
+// scalar field (NIN = RED_SCAL, input 0) or one vector's length (NIN = RED_VEC,
+// inputs 0-2); sets 1 .. NS-1 are the scalar fields of the inputs that follow
 // (input s for a scalar request, s - 1 for a vector one): the vector's
 // components and, in the single-precision builds, the fields that share their
-// 8-byte elements, whose bytes the pass reads anyway. Every set's accumulators
-// are combined in exactly the order reduce3_kernel combines its three, so each
-// set's results equal a reduce3_kernel pass over it, bit for bit. partials
-// holds 3 * NS * gridDim.x doubles, result 3 * NS (set s at 3 s).
+// 8-byte elements (input NIN + w that of input w), whose bytes the pass reads
+// anyway. Every set's accumulators are combined in the order in which
+// reduce_kernel combines its one, so each equals a pass of its own, bit for bit;
+// a vector's MAX and MIN are kept as |v|^2 until the end (sqrt is monotonic and
+// correctly rounded, so the root of the largest square is the largest length).
+// partials holds 3 * NS * gridDim.x doubles, result 3 * NS (set s at 3 s).
 template <int THREADS, int NIN, int NS>
 __global__ void __launch_bounds__(THREADS)
 reduce_sets_kernel(const ReduceArgs a)
 {
     constexpr int NF = NIN == RED_SCAL ? NS : (NS - 1 > 3 ? NS - 1 : 3); // inputs
     static_assert(NF <= 6, "at most six inputs");
-    const Layout& L = a.L;
-    const int lane  = threadIdx.x & 31;
-    const int wid   = threadIdx.x >> 5;
-    const long long gw  = ((long long)blockIdx.x * THREADS + threadIdx.x) >> 5;
-    const long long nw  = ((long long)gridDim.x * THREADS) >> 5;
-    const int rx        = a.end.x - a.start.x;
-    const int ry        = a.end.y - a.start.y;
+    const int lane = threadIdx.x & 31;
+    const int wid  = threadIdx.x >> 5;
     double mx[NS], mn[NS], sm[NS];
 #pragma unroll
     for (int t = 0; t < NS; ++t) {
@@ -305,23 +280,24 @@ reduce_sets_kernel(const ReduceArgs a)
         mn[t] = INFINITY;
         sm[t] = 0.0;
     }
-    for (long long r = gw; r < a.rows; r += nw) {
-        const int j          = a.start.y + (int)(r % ry);
-        const int k          = a.start.z + (int)(r / ry);
-        const long long base = lidx(L, a.start.x, j, k);
-        for (int i = lane; i < rx; i += 32) {
-            const long long id = base + i;
-            double v[NF];
+    red_rows<THREADS, NF>(
+        a,
+        [&](long long id, double* v) {
+            if (ACB_PAIRED && NF == 2 * NIN)
 #pragma unroll
-            for (int w = 0; w < NF; ++w)
-                v[w] = red_load(a, w, id);
+                for (int w = 0; w < NIN; ++w)
+                    red_load_pair(a, w, id, v[w], v[NIN + w]);
+            else
+#pragma unroll
+                for (int w = 0; w < NF; ++w)
+                    v[w] = red_load(a, w, id);
+        },
+        [&](const double* v) {
 #pragma unroll
             for (int t = 0; t < NS; ++t) {
                 double m, q;
-                if (t == 0 && NIN == RED_VEC) {
-                    q = red_len2(v[0], v[1], v[2]);
-                    m = sqrt(q);
-                }
+                if (t == 0 && NIN == RED_VEC)
+                    m = q = red_len2(v[0], v[1], v[2]);
                 else {
                     m = v[NIN == RED_SCAL ? t : t - 1];
                     q = __dmul_rn(m, m);
@@ -330,8 +306,7 @@ reduce_sets_kernel(const ReduceArgs a)
                 mn[t] = fmin(mn[t], m);
                 sm[t] = sm[t] + q;
             }
-        }
-    }
+        });
 #pragma unroll
     for (int t = 0; t < NS; ++t)
 #pragma unroll
@@ -400,9 +375,15 @@ reduce_sets_kernel(const ReduceArgs a)
                     bn = fmin(bn, wmn[t][w]);
                     bs = bs + wsm[t][w];
                 }
+                if (t == 0 && NIN == RED_VEC) { // (an identity stays one)
+                    bx = bx < 0.0 ? bx : sqrt(bx);
+                    bn = sqrt(bn);
+                }
                 a.result[3 * t]     = bx;
                 a.result[3 * t + 1] = bn;
                 a.result[3 * t + 2] = bs;
+                if (t == 0 && a.cfl_rec)
+                    cfl_step(bx, a.cfl, a.cfl_rec);
             }
             *a.counter = 0u; // ready for the next launch on this stream
         }
