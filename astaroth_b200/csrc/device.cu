@@ -14,6 +14,7 @@
 //     instead of one __constant__ AcMeshInfo per GPU; loads keep the
 //     reference's rule of skipping NaN/inf values with a warning;
 //   - reductions use per-device FP64 scratch of one double per CTA.
+#include <limits.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -34,9 +35,9 @@ const SolveConfig*
 acb_host::solve_configs(int* n)
 {
     static const SolveConfig table[] = {
-        make_solve_config<SolveCfg0, false>(),
-        make_solve_config<SolveCfg1, false>(),
-        make_solve_config<SolveCfg2, false>(),
+        make_solve_config<SolveCfg0, false>(kPlaneCost[0]),
+        make_solve_config<SolveCfg1, false>(kPlaneCost[1]),
+        make_solve_config<SolveCfg2, false>(kPlaneCost[2]),
     };
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;
@@ -393,26 +394,122 @@ acb_host::make_params(const AcMeshInfo& uniforms, const Layout& L, int step, int
     return P;
 }
 
-// Cuts z into 1..8 segments of at least `min_planes` planes so that the last
-// wave of (tile, segment) tasks is as full as possible; fewer segments win
-// near-ties because each segment re-reads 6 halo planes.
-int
-acb_host::choose_segments(long long ntiles, int nzr, long long slots, int min_planes)
+// Splits the tile columns of a launch over at most `slots` CTAs (SolveGeom's
+// nfull ... left, see Pieces) and returns the grid. A CTA's time is counted in
+// planes: its planes plus piece_cost for each piece, the time a piece takes to
+// fill its ring and prime its queues before its first output. The split is the
+// one with the smallest score, the time of the longest CTA plus the average over
+// the SMs: the former is what a mesh alone waits for, the latter what several in
+// flight share. Two forms compete:
+//   - whole columns, and the rem < slots columns of the last wave cut into slabs;
+//     what the slabs leave is shared by the CTAs that have none (at staggered z,
+//     where neighbours share fewer halos in L2: 4 % dearer, and 1 % for what runs
+//     beside it, the mixed build's 192^3 and 512^3 steps as measured);
+//   - uniform z segments, dealt in several rounds.
+// Against uniform segments of at least 16 planes alone, a step of a 32^3 FP32 mesh
+// takes 29 us instead of 102, 64^3 57 instead of 107, 112^3 200 instead of 205 (FP64
+// 39, 91 and 352 instead of 139, 147 and 382).
+static int
+split_columns(SolveGeom& g, int slots, double piece_cost, double* score)
 {
-    int best_seg    = 1;
-    double best_eff = -1.0;
-    for (int ns = 1; ns <= 8; ++ns) {
-        if (ns > 1 && nzr / ns < min_planes)
-            break;
-        const long long T    = ntiles * ns;
-        const long long wave = (T + slots - 1) / slots;
-        const double eff     = (double)T / (double)(wave * slots) - 0.01 * (ns - 1);
-        if (eff > best_eff + 1e-9) {
-            best_eff = eff;
-            best_seg = ns;
+    const long long ntiles = (long long)g.ntx * g.nty;
+    const int nz           = g.nzr;
+    g.nfull                = (int)(ntiles / slots);
+    g.rem0                 = g.nfull * slots;
+    g.rem                  = (int)(ntiles - g.rem0);
+    g.slabs = g.slab_planes = g.left = g.zseg = g.seg_tasks = 0;
+    const double full = g.nfull * (nz + piece_cost);
+    double best       = INFINITY;
+    auto better       = [&](double t) {
+        if (!(t < best))
+            return false;
+        best = t;
+        return true;
+    };
+    if (g.rem == 0)
+        better(2.0 * full);
+    for (int k = 1; g.rem > 0 && k <= slots / g.rem && k <= nz; ++k) {
+        const int others = slots - k * g.rem; // CTAs without a slab
+        for (int q = nz / (k + 1) + 1; q <= (nz + k - 1) / k; ++q) {
+            const int left = std::max(0, nz - k * q);
+            if (left > 0 && others == 0)
+                continue;
+            double t      = q + piece_cost;
+            double pieces = k * (double)g.rem;
+            if (left > 0) {
+                const double cols = (double)g.rem / others; // columns per CTA
+                t = std::max(t, ceil(cols * left) + piece_cost * (ceil(cols) + 1.0));
+                pieces += others + g.rem;
+            }
+            const double mean = ((double)g.rem * nz + piece_cost * pieces) / slots;
+            if (better(left > 0 ? 1.01 * (2.0 * full + 1.03 * (t + mean))
+                                : 2.0 * full + t + mean)) {
+                g.slabs       = k;
+                g.slab_planes = q;
+                g.left        = left;
+            }
         }
     }
-    return best_seg;
+    for (int ns = 2; ns <= 8 && nz / ns >= 16; ++ns) {
+        const int zseg         = (nz + ns - 1) / ns;
+        const long long tasks  = ntiles * ((nz + zseg - 1) / zseg);
+        const long long rounds = (tasks + slots - 1) / slots;
+        if (tasks < slots || tasks > INT_MAX)
+            continue; // (slabs)
+        const double mean      = (ntiles * nz + piece_cost * tasks) / slots;
+        if (better(rounds * (zseg + piece_cost) + mean)) {
+            g.zseg      = zseg;
+            g.seg_tasks = (int)tasks;
+        }
+    }
+    *score = best;
+    if (g.seg_tasks > 0 || g.nfull > 0 || g.left > 0)
+        return slots;
+    return g.slabs * g.rem;
+}
+
+// Time of starting a piece, in planes of the first configuration's tile (FP32: a
+// substep takes about 6 us, launch included, and 1.65 us per plane of its longest
+// CTA).
+constexpr double kPieceCost = 3.0;
+
+// The tiles of a launch over the box [s, e) and their split over the CTAs.
+static int
+solve_geometry(const SolveConfig& cfg, const Layout& L, int3 s, int3 e, int slots, SolveGeom& g,
+               double* score)
+{
+    g.L     = L;
+    g.start = s;
+    g.end   = e;
+    g.tx0   = (s.x - NGHOST) / cfg.TX;
+    g.ntx   = (e.x - 1 - NGHOST) / cfg.TX - g.tx0 + 1;
+    g.nty   = (e.y - s.y + cfg.TY - 1) / cfg.TY;
+    g.nzr   = e.z - s.z;
+    return split_columns(g, slots, kPieceCost / cfg.plane_cost, score);
+}
+
+// The tile configuration with which a mesh's substep takes least time: the score
+// of its split (split_columns), in planes, times what a plane costs (plane_cost).
+// Large meshes take the largest tile, which reads least halo; a small one whose
+// rows or columns fill another better takes that.
+static int
+default_config(const Layout& L, int num_sms)
+{
+    int n, best = kDefaultSolveConfig;
+    const SolveConfig* cfgs = solve_configs(&n);
+    double least            = INFINITY;
+    for (int c = 0; c < n; ++c) {
+        SolveGeom g;
+        double score;
+        solve_geometry(cfgs[c], L, make_int3(NGHOST, NGHOST, NGHOST),
+                       make_int3(NGHOST + L.nx, NGHOST + L.ny, NGHOST + L.nz),
+                       num_sms, g, &score);
+        if (score * cfgs[c].plane_cost < least) {
+            least = score * cfgs[c].plane_cost;
+            best  = c;
+        }
+    }
+    return best;
 }
 
 static bool
@@ -447,13 +544,6 @@ launch_solve(const Device d, cudaStream_t st, int step, int3 s, int3 e,
     SolveArgs<AcReal> a;
     memset(&a, 0, sizeof(a));
     SolveGeom& g = a.g;
-    g.L          = d->L;
-    g.start      = s;
-    g.end        = e;
-    g.tx0        = (s.x - NGHOST) / cfg.TX;
-    g.ntx        = (e.x - 1 - NGHOST) / cfg.TX - g.tx0 + 1;
-    g.nty        = (e.y - s.y + cfg.TY - 1) / cfg.TY;
-    g.nzr        = e.z - s.z;
     a.out        = d->blk[d->cur ^ 1];
     a.in_lo      = d->lo[d->cur];
     a.out_lo     = d->lo[d->cur ^ 1];
@@ -481,17 +571,11 @@ launch_solve(const Device d, cudaStream_t st, int step, int3 s, int3 e,
                                                                  cfg.threads, cfg.smem));
     if (per_sm < 1)
         per_sm = 1;
-    const long long slots = (long long)d->num_sms * per_sm;
-    const long long ntiles = (long long)g.ntx * g.nty;
-    const int best_seg     = choose_segments(ntiles, g.nzr, slots, 16);
-    g.nseg  = best_seg;
-    g.zseg  = (g.nzr + best_seg - 1) / best_seg;
-    g.nseg  = (g.nzr + g.zseg - 1) / g.zseg;
-    g.tasks = ntiles * g.nseg;
-    long long grid = std::min(slots, g.tasks);
+    double score;
+    const int grid = solve_geometry(cfg, d->L, s, e, d->num_sms * per_sm, g, &score);
     if (diag) {
         if (grid > d->diag_max_ctas) {
-            fprintf(stderr, "astaroth_b200: %lld CTAs exceed the step diagnostics' %d partials\n",
+            fprintf(stderr, "astaroth_b200: %d CTAs exceed the step diagnostics' %d partials\n",
                     grid, d->diag_max_ctas);
             return AC_FAILURE;
         }
@@ -1389,7 +1473,6 @@ acDeviceCreate(const int id, const AcMeshInfo config, Device* device_handle)
     d->id           = id;
     d->local_config = config;
     d->tmap_cfg     = -1;
-    d->solve_cfg    = kDefaultSolveConfig;
     ACB_CUDA_CHECK(cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, id));
 
     int prio_lo = 0, prio_hi = 0;
@@ -1402,6 +1485,7 @@ acDeviceCreate(const int id, const AcMeshInfo config, Device* device_handle)
     }
 
     d->L               = make_layout(nx, ny, nz);
+    d->solve_cfg       = default_config(d->L, d->num_sms);
     const size_t bytes = block_bytes(d->L);
     for (int b = 0; b < 2; ++b) {
         ACB_CUDA_CHECK(cudaMalloc((void**)&d->blk[b], bytes));
@@ -2021,7 +2105,7 @@ acDeviceSetSolveConfig(const Device device, const int config)
 {
     int n;
     solve_configs(&n);
-    const int c = config < 0 ? kDefaultSolveConfig : config;
+    const int c = config < 0 ? default_config(device->L, device->num_sms) : config;
     if (c >= n)
         return AC_FAILURE;
     if (device->solve_cfg != c) {

@@ -6,9 +6,10 @@
 // holds one __constant__ parameter block, src/core/kernels/kernels.cu:9).
 //
 // Members keep the Device layout (common.cuh: Layout) and the solve kernel of
-// solve.cuh in its ensemble form: each (tile, z segment) task finds its member
-// in a descriptor table in global memory (TMA map, geometry, buffers,
-// parameters), one table per buffer parity.
+// solve.cuh in its ensemble form: each CTA marches a list of pieces (planes of
+// one tile column of one member) made here, and finds a piece's member in a
+// descriptor table in global memory (TMA map, geometry, buffers), one table per
+// buffer parity.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -32,9 +33,9 @@ const SolveConfig*
 acb_host::ensemble_configs(int* n)
 {
     static const SolveConfig table[] = {
-        make_solve_config<SolveCfg0, true>(),
-        make_solve_config<SolveCfg1, true>(),
-        make_solve_config<SolveCfg2, true>(),
+        make_solve_config<SolveCfg0, true>(kPlaneCost[0]),
+        make_solve_config<SolveCfg1, true>(kPlaneCost[1]),
+        make_solve_config<SolveCfg2, true>(kPlaneCost[2]),
     };
     *n = (int)(sizeof(table) / sizeof(table[0]));
     return table;
@@ -93,6 +94,7 @@ struct ensemble_s {
     int cur; // buffer parity: blk[cur] is `in` for every member
     int cfg;
     int seg_planes; // target planes per z segment (0: whole columns)
+    bool seg_given; // set by the caller or the tuner (else whole columns)
     // ghost_ok[p]: the ghosts of every member's block p hold periodic images
     bool ghost_ok[2];
     StageBuf stage; // staging buffer of member loads
@@ -106,8 +108,15 @@ struct ensemble_s {
     MemberDesc<AcReal>* d_desc[2];
     HaloMember* d_halo[2];
     long long halo_total; // work units of one batched ghost fill
-    long long total_tasks;
-    int grid;
+    // the schedule: one launch per group of ACB_ENS_GROUP members, each with its
+    // CTAs' pieces and their first ones in device memory
+    struct Group {
+        int grid;
+        Piece* pieces;
+        int* first;
+    };
+    std::vector<Group> groups;
+    void* d_schedule; // one allocation for all groups
 
     unsigned long long launches;
     unsigned long long version; // bumped on any schedule change
@@ -131,8 +140,72 @@ drop_graphs(Ensemble e)
     }
 }
 
-// (Re)builds both parities' descriptor tables and ghost-fill tables for the
-// current tile configuration and segment length, and uploads them.
+// Splits the units (whole columns, or z segments of them; longest first) of one
+// launch over `slots` CTAs. Full rounds of units are dealt round-robin, so that
+// the CTAs of a round stream neighbouring tiles at the same z and share their
+// halos in L2. With `level`, the units of the last, partial round are cut so
+// that all CTAs end together, counting kPieceCost planes for each piece (the
+// time to fill its ring and prime its queues): the CTAs take the units' first
+// planes in step, as many units as there are CTAs at a time, and the CTAs left
+// over share what remains of the units, running from one to the next. Without
+// it they go to one CTA each. (64 FP32 meshes of 32^3 ... 128^3: 0.7 % of a step
+// against z segments of 32 planes dealt round-robin.)
+void
+schedule(const std::vector<Piece>& units, int slots, bool level,
+         std::vector<std::vector<Piece>>& cta)
+{
+    constexpr int kPieceCost = 2;
+    cta.assign(slots, {});
+    std::vector<int> load(slots, 0);
+    const int n = (int)units.size(), full = n / slots * slots, rem = n - full;
+    for (int i = 0; i < (level ? full : n); ++i) {
+        cta[i % slots].push_back(units[i]);
+        load[i % slots] += units[i].n + kPieceCost;
+    }
+    if (!level || rem == 0)
+        return;
+    long long sum = 0;
+    for (int c = 0; c < slots; ++c)
+        sum += load[c];
+    for (int i = full; i < n; ++i)
+        sum += units[i].n;
+    std::vector<std::vector<Piece>> tail;
+    for (long long T = (sum + slots - 1) / slots + kPieceCost;; T += std::max(1LL, T / 256)) {
+        tail.assign(slots, {});
+        std::vector<Piece> left(units.begin() + full, units.end());
+        auto take = [&](int c, Piece& u, long long room) {
+            const int m = (int)std::min<long long>(u.n, room);
+            if (m <= 0)
+                return 0;
+            Piece p = u;
+            p.n     = m;
+            tail[c].push_back(p);
+            u.z0 += m;
+            u.n -= m;
+            return m;
+        };
+        const int in_step = slots / rem * rem;
+        for (int c = 0; c < in_step; ++c)
+            take(c, left[c % rem], T - load[c] - kPieceCost);
+        int i = 0;
+        for (int c = in_step; c < slots; ++c)
+            for (long long room = T - load[c] - kPieceCost; room > 0 && i < rem;) {
+                room -= take(c, left[i], room) + kPieceCost;
+                if (left[i].n == 0)
+                    ++i;
+            }
+        while (i < rem && left[i].n == 0)
+            ++i;
+        if (i == rem)
+            break;
+    }
+    for (int c = 0; c < slots; ++c)
+        cta[c].insert(cta[c].end(), tail[c].begin(), tail[c].end());
+}
+
+// (Re)builds both parities' descriptor tables and ghost-fill tables and the
+// schedule for the current tile configuration and segment length, and uploads
+// them.
 AcResult
 build_tables(Ensemble e)
 {
@@ -147,27 +220,26 @@ build_tables(Ensemble e)
                                                                  cfg.smem));
     per_sm = std::max(per_sm, 1);
     e->h_mp.assign(n, RhsParams<AcReal>());
+    const int seg_planes = e->seg_given ? e->seg_planes : 0;
+    // planes per unit of a member: its z range in equal segments
+    auto zseg_of = [&](const Layout& L) {
+        int nseg = 1;
+        if (seg_planes > 0)
+            nseg = std::max(1, (int)lround((double)L.nz / seg_planes));
+        return (L.nz + nseg - 1) / nseg;
+    };
+    // members with the longest units first
+    std::vector<int> order(n);
+    for (int i = 0; i < n; ++i)
+        order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return zseg_of(e->m[a].L) > zseg_of(e->m[b].L);
+    });
     for (int p = 0; p < 2; ++p) {
         std::vector<MemberDesc<AcReal>>& D = e->h_desc[p];
         D.assign(n, MemberDesc<AcReal>());
         std::vector<HaloMember> H(n);
-        long long tasks = 0, units = 0;
-        // Task list order: members with the longest tasks (z segment + halo
-        // planes) first, so that the persistent CTAs, which take tasks
-        // round-robin, finish the launch on short tasks instead of idling
-        // behind a few long ones (longest-processing-time-first).
-        auto zseg_of = [&](const Layout& L) {
-            int nseg = 1;
-            if (e->seg_planes > 0)
-                nseg = std::max(1, (int)lround((double)L.nz / e->seg_planes));
-            return (L.nz + nseg - 1) / nseg;
-        };
-        std::vector<int> order(n);
-        for (int i = 0; i < n; ++i)
-            order[i] = i;
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-            return zseg_of(e->m[a].L) > zseg_of(e->m[b].L);
-        });
+        long long units = 0;
         for (int pos = 0; pos < n; ++pos) {
             const int i      = order[pos];
             const Member& mb = e->m[i];
@@ -184,11 +256,6 @@ build_tables(Ensemble e)
             g.ntx        = (L.nx + cfg.TX - 1) / cfg.TX;
             g.nty        = (L.ny + cfg.TY - 1) / cfg.TY;
             g.nzr        = L.nz;
-            g.zseg        = zseg_of(L);
-            g.nseg        = (L.nz + g.zseg - 1) / g.zseg;
-            g.tasks       = (long long)g.ntx * g.nty * g.nseg;
-            d.task_begin  = tasks;
-            tasks += g.tasks;
             d.out         = mb.blk[p ^ 1];
             d.in_lo       = mb.lo[p];
             d.out_lo      = mb.lo[p ^ 1];
@@ -200,14 +267,57 @@ build_tables(Ensemble e)
             H[pos].units_a    = (unsigned)halo_units_a(L);
             units += halo_units(L);
         }
-        e->total_tasks = tasks;
         e->halo_total  = units;
         ACB_CUDA_CHECK(cudaMemcpy(e->d_desc[p], D.data(), sizeof(MemberDesc<AcReal>) * n,
                                   cudaMemcpyHostToDevice));
         ACB_CUDA_CHECK(cudaMemcpy(e->d_halo[p], H.data(), sizeof(HaloMember) * n,
                                   cudaMemcpyHostToDevice));
     }
-    e->grid       = (int)std::min<long long>((long long)e->num_sms * per_sm, e->total_tasks);
+    // the schedule: all groups' pieces, then all groups' first ones
+    std::vector<Piece> pieces;
+    std::vector<int> first;
+    std::vector<size_t> piece_at, first_at;
+    e->groups.clear();
+    for (int g0 = 0; g0 < n; g0 += ACB_ENS_GROUP) {
+        std::vector<Piece> units;
+        for (int pos = g0; pos < std::min(n, g0 + ACB_ENS_GROUP); ++pos) {
+            const SolveGeom& g = e->h_desc[0][pos].g;
+            const int zseg     = zseg_of(g.L);
+            for (int z0 = 0; z0 < g.nzr; z0 += zseg)
+                for (int t = 0; t < g.ntx * g.nty; ++t)
+                    units.push_back(Piece{t, z0, std::min(zseg, g.nzr - z0), pos - g0});
+        }
+        std::vector<std::vector<Piece>> cta;
+        schedule(units, e->num_sms * per_sm, seg_planes == 0, cta);
+        piece_at.push_back(pieces.size());
+        first_at.push_back(first.size());
+        int grid = 0, at = 0;
+        for (const auto& list : cta) {
+            if (list.empty())
+                continue;
+            first.push_back(at);
+            pieces.insert(pieces.end(), list.begin(), list.end());
+            at += (int)list.size();
+            ++grid;
+        }
+        first.push_back(at);
+        e->groups.push_back({grid, nullptr, nullptr});
+    }
+    if (e->d_schedule)
+        cudaFree(e->d_schedule);
+    e->d_schedule = nullptr;
+    ACB_CUDA_CHECK(cudaMalloc(&e->d_schedule,
+                              pieces.size() * sizeof(Piece) + first.size() * sizeof(int)));
+    Piece* dp = (Piece*)e->d_schedule;
+    int* df   = (int*)(dp + pieces.size());
+    ACB_CUDA_CHECK(cudaMemcpy(dp, pieces.data(), pieces.size() * sizeof(Piece),
+                              cudaMemcpyHostToDevice));
+    ACB_CUDA_CHECK(cudaMemcpy(df, first.data(), first.size() * sizeof(int),
+                              cudaMemcpyHostToDevice));
+    for (size_t g = 0; g < e->groups.size(); ++g) {
+        e->groups[g].pieces = dp + piece_at[g];
+        e->groups[g].first  = df + first_at[g];
+    }
     e->desc_valid = true;
     drop_graphs(e);
     return AC_SUCCESS;
@@ -247,17 +357,14 @@ launch_solve_all(Ensemble e, cudaStream_t st, int step, AcReal dt)
     // ensemble kernels take their centre values by plain loads: no centre maps
     static const CentreMaps no_centre_maps = {};
     const std::vector<MemberDesc<AcReal>>& D = e->h_desc[e->cur];
-    for (int g0 = 0; g0 < n; g0 += ACB_ENS_GROUP) {
-        const int gn            = std::min(ACB_ENS_GROUP, n - g0);
-        const long long t_begin = D[g0].task_begin;
-        const long long t_end   = g0 + gn < n ? D[g0 + gn].task_begin : e->total_tasks;
-        a.members               = e->d_desc[e->cur] + g0;
-        a.nmembers              = gn;
-        a.task_base             = t_begin;
-        a.total_tasks           = t_end - t_begin;
+    for (size_t g = 0; g < e->groups.size(); ++g) {
+        const int g0 = (int)g * ACB_ENS_GROUP, gn = std::min(ACB_ENS_GROUP, n - g0);
+        a.members    = e->d_desc[e->cur] + g0;
+        a.pieces     = e->groups[g].pieces;
+        a.first      = e->groups[g].first;
         for (int i = 0; i < gn; ++i)
             a.mp[i] = e->h_mp[g0 + i];
-        const int grid = (int)std::min<long long>(e->grid, a.total_tasks);
+        const int grid = e->groups[g].grid;
         // the map parameter is not read in ensemble mode; any valid map fills it
         ((EnsKernelFn)cfg.kern[step])<<<grid, cfg.threads, cfg.smem, st>>>(D[0].tmap, a,
                                                                            no_centre_maps);
@@ -424,6 +531,8 @@ acEnsembleDestroy(Ensemble e)
         if (e->d_halo[p])
             cudaFree(e->d_halo[p]);
     }
+    if (e->d_schedule)
+        cudaFree(e->d_schedule);
     if (e->status)
         cudaFree(e->status);
     stage_destroy(&e->stage);
@@ -565,6 +674,7 @@ acEnsembleSetSchedule(Ensemble e, const int config, const int segment_planes)
     ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     e->cfg        = config;
     e->seg_planes = segment_planes;
+    e->seg_given  = true;
     e->version++;
     return build_tables(e);
 }

@@ -32,6 +32,17 @@ using SolveCfg1 = TileCfg<32, 8, 9, 1>;
 using SolveCfg2 = TileCfg<64, 6, 7, 1>;
 #endif
 
+// Time of a plane of each configuration's tile relative to the first's (256^3
+// steps, in planes of the longest CTA: FP32 1621, 1649 and 1667 us, mixed 1930,
+// 2001 and 2049 us, FP64 3523, 3993 and 4231 us).
+#if AC_DOUBLE_PRECISION == 1
+constexpr double kPlaneCost[3] = {1.0, 0.845, 0.60};
+#elif ACB_MIXED
+constexpr double kPlaneCost[3] = {1.0, 0.715, 0.73};
+#else
+constexpr double kPlaneCost[3] = {1.0, 0.70, 1.05};
+#endif
+
 typedef void (*SolveKernelFn)(const CUtensorMap, const SolveArgs<AcReal>, const CentreMaps);
 typedef void (*EnsKernelFn)(const CUtensorMap, const EnsSolveArgs<AcReal>, const CentreMaps);
 
@@ -41,6 +52,7 @@ struct SolveConfig {
     int launch_regs; // registers a thread the kernels must be launched with (0: any)
     int NC;          // centre ring slots (0: the centre values are plain loads)
     size_t smem;
+    double plane_cost; // time of one plane of a tile, relative to the first configuration's
     // substeps 0, 1, 2, and 2 with helical forcing (single mesh only): a
     // SolveKernelFn, or an EnsKernelFn in the ensemble table
     const void* kern[4];
@@ -67,7 +79,7 @@ solve_config_name()
 
 template <class Cfg, bool ENS>
 SolveConfig
-make_solve_config()
+make_solve_config(double plane_cost)
 {
     SolveConfig c;
     c.name    = solve_config_name<Cfg, ENS>();
@@ -75,6 +87,7 @@ make_solve_config()
     c.TY      = Cfg::TY;
     c.NP      = Cfg::NP;
     c.threads = Cfg::THREADS;
+    c.plane_cost  = plane_cost;
     c.launch_regs = Cfg::REG_LAUNCH;
     c.NC          = ENS ? 0 : Cfg::NC;
     c.smem    = ENS ? Cfg::ring_bytes() : Cfg::smem_bytes(); // ensembles load centres directly
@@ -121,9 +134,6 @@ AcResult encode_centre_map(const Layout& L, const void* block, const SolveConfig
 // and rounded once to AcReal; rkA/rkB for `step` from AC_dt
 SolveParams<AcReal> make_params(const AcMeshInfo& uniforms, const Layout& L, int step,
                                 int forcing);
-
-// z segments per tile column so that tiles*segments fills the last wave best
-int choose_segments(long long ntiles, int nzr, long long slots, int min_planes);
 
 // Device staging buffer of loads and stores: the caller's values pass through
 // it in one contiguous transfer per chunk, and a kernel scatters them into (or

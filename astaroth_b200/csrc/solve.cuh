@@ -14,9 +14,10 @@
 //
 // B200 structure (no counterpart in the reference, which reads 55 stencil points
 // per field straight from global memory with one thread per vertex):
-//   - persistent CTAs (one per SM slot) take tasks = (x-y tile, z segment)
-//     round-robin, segment-major, so the CTAs of one wave stream neighbouring
-//     tiles at the same z and read each other's halo planes from L2;
+//   - persistent CTAs (one per SM slot) march the columns of x-y tiles
+//     round-robin, so the CTAs of one wave stream neighbouring tiles at the same
+//     z and read each other's halo planes from L2, and share the planes of the
+//     last, partial wave evenly (Pieces; ensembles: a list made by the host);
 //   - each CTA streams its tile along z (2.5D): a producer warp issues one TMA
 //     load per plane bringing all eight fields of a (TX+8) x (TY+6) halo'd tile
 //     into a ring of NP plane slots in shared memory (mbarrier `full` with
@@ -92,9 +93,21 @@ struct SolveGeom {
                      // so that every TMA box starts on a 16-byte boundary
     int ntx, nty;    // tiles covering the region
     int nzr;         // planes of the region
-    int zseg;        // planes per task (the region's z range is cut into nseg segments)
-    int nseg;
-    long long tasks; // ntx * nty * nseg; task t = (segment t / tiles, tile t % tiles)
+    // single mesh: each CTA marches `nfull` whole columns, tiles blockIdx.x +
+    // w * gridDim.x; the `rem` tiles left (from tile `rem0`) are cut into
+    // `slabs` slabs of `slab_planes` planes, one CTA per tile and slab, and the
+    // last `left` planes of each are shared by the other CTAs (see Pieces)
+    int nfull, rem0, rem;
+    int slabs, slab_planes, left;
+    // or (seg_tasks > 0) the columns are cut into segments of zseg planes, dealt
+    // round-robin: task t = (segment t / tiles, tile t % tiles)
+    int zseg, seg_tasks;
+};
+
+// One task of a CTA: planes [z0, z0 + n) of the column of one x-y tile (of one
+// member, by its position in the descriptor table, in an ensemble).
+struct __align__(16) Piece {
+    int tile, z0, n, member;
 };
 
 // One member of an ensemble (many independent meshes advanced by one launch):
@@ -105,7 +118,6 @@ template <typename T>
 struct __align__(128) MemberDesc {
     CUtensorMap tmap;
     SolveGeom g;
-    long long task_begin; // first global task of this member (tasks are member-major)
     state_t* out;
     lo16_t* in_lo;
     lo16_t* out_lo;
@@ -127,8 +139,6 @@ struct SolveArgs {
     double* diag_result;
     // ensemble launches only
     const MemberDesc<T>* members;
-    int nmembers;
-    long long total_tasks;
 };
 
 // Members per ensemble launch (a launch's parameters stay within 32 KB; a
@@ -137,8 +147,10 @@ constexpr int ACB_ENS_GROUP = 64;
 
 template <typename T>
 struct EnsSolveArgs : SolveArgs<T> {
-    long long task_base;                 // first task of the group (tasks of all groups
-                                         // are numbered as one list, member-major)
+    // the pieces of the group's members that CTA b marches, in order:
+    // pieces[first[b]] ... pieces[first[b + 1] - 1]
+    const Piece* pieces;
+    const int* first;
     RhsParams<T> mp[ACB_ENS_GROUP];      // by position in the group
 };
 
@@ -1040,19 +1052,107 @@ prefetch_centre2(const Layout& L, const state_t* out, const lo16_t* in_lo, const
     (void)ol;
 }
 
+// The pieces of a single mesh that this CTA marches, in order: its whole columns,
+// dealt round-robin so that the CTAs stream neighbouring tiles at the same z and
+// read each other's halos from L2; then its part of the last, partial wave (all
+// there is on a mesh of fewer tiles than CTAs), a slab of one column or an even
+// share, running from column to column, of the planes below the slabs' end.
+struct Pieces {
+    int w, p, pend;
+    __device__ __forceinline__ Pieces(const SolveGeom& g)
+    {
+        if (g.seg_tasks > 0) {
+            p    = blockIdx.x;
+            pend = g.seg_tasks;
+            return;
+        }
+        w                = 0;
+        const int nslab  = g.slabs * g.rem; // CTAs with a slab
+        const int b      = (int)blockIdx.x - nslab, n = (int)gridDim.x - nslab;
+        const long long planes = (long long)g.rem * g.left;
+        p    = b < 0 ? 0 : (int)(planes * b / n);
+        pend = b < 0 ? 1 : (int)(planes * (b + 1) / n); // a slab: one piece
+    }
+    __device__ __forceinline__ bool next(const SolveGeom& g, Piece& r)
+    {
+        if (g.seg_tasks > 0) {
+            if (p >= pend)
+                return false;
+            const int tiles = g.ntx * g.nty, seg = p / tiles;
+            r.tile          = p - seg * tiles;
+            r.z0            = seg * g.zseg;
+            r.n             = min(g.zseg, g.nzr - r.z0);
+            p += (int)gridDim.x;
+            return true;
+        }
+        if (w < g.nfull) {
+            r.tile = (int)(blockIdx.x + (unsigned)w * gridDim.x);
+            r.z0   = 0;
+            r.n    = g.nzr;
+            ++w;
+            return true;
+        }
+        if (p >= pend)
+            return false;
+        const int b = (int)blockIdx.x;
+        if (b < g.slabs * g.rem) {
+            const int s = b / g.rem;
+            r.tile      = g.rem0 + (b - s * g.rem);
+            r.z0        = s * g.slab_planes;
+            r.n         = min(g.slab_planes, g.nzr - r.z0);
+            p           = pend;
+            return r.n > 0;
+        }
+        const int col = p / g.left;
+        r.tile        = g.rem0 + col;
+        r.z0          = g.nzr - g.left + (p - col * g.left);
+        r.n           = min(g.nzr - r.z0, pend - p);
+        p += r.n;
+        return true;
+    }
+};
+
+// The pieces of this CTA: of a single mesh, or an ensemble's listed ones.
+template <bool ENS>
+struct PieceList : Pieces {
+    __device__ __forceinline__ PieceList(const SolveArgs<AcReal>& a) : Pieces(a.g) {}
+    __device__ __forceinline__ bool next(const SolveArgs<AcReal>& a, Piece& r)
+    {
+        return Pieces::next(a.g, r);
+    }
+};
+template <>
+struct PieceList<true> {
+    int p, pend;
+    __device__ __forceinline__ PieceList(const EnsSolveArgs<AcReal>& a)
+    {
+        p    = a.first[blockIdx.x];
+        pend = a.first[blockIdx.x + 1];
+    }
+    __device__ __forceinline__ bool next(const EnsSolveArgs<AcReal>& a, Piece& r)
+    {
+        if (p >= pend)
+            return false;
+        const int4 v = reinterpret_cast<const int4*>(a.pieces)[p++];
+        r.tile       = v.x;
+        r.z0         = v.y;
+        r.n          = v.z;
+        r.member     = v.w;
+        return true;
+    }
+};
+
 template <class Cfg>
 struct TaskGeom {
     int i0, j0, k0, nout;
-    __device__ __forceinline__ TaskGeom(const SolveGeom& g, long long t, long long ntiles)
+    __device__ __forceinline__ TaskGeom(const SolveGeom& g, const Piece& p)
     {
-        const long long seg  = t / ntiles;
-        const long long tile = t - seg * ntiles;
-        const int tile_x     = (int)(tile % g.ntx);
-        const int tile_y     = (int)(tile / g.ntx);
-        i0                   = NGHOST + (g.tx0 + tile_x) * Cfg::TX;
-        j0                   = g.start.y + tile_y * Cfg::TY;
-        k0                   = g.start.z + (int)seg * g.zseg;
-        nout                 = min(g.zseg, g.nzr - (int)seg * g.zseg);
+        const int tile_y = p.tile / g.ntx;
+        const int tile_x = p.tile - tile_y * g.ntx;
+        i0               = NGHOST + (g.tx0 + tile_x) * Cfg::TX;
+        j0               = g.start.y + tile_y * Cfg::TY;
+        k0               = g.start.z + p.z0;
+        nout             = p.n;
     }
 };
 
@@ -1064,30 +1164,13 @@ fence_tensormap_acquire(const CUtensorMap* map)
                  : "memory");
 }
 
-// Which member an ensemble task belongs to (binary search on task_begin).
-template <typename T>
-__device__ __forceinline__ int
-member_of(const MemberDesc<T>* md, int n, long long t)
-{
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (md[mid].task_begin <= t)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
-
 // One task of a consumer warp: the planes of one (tile, z segment) column.
 // Waits for the ring, computes and stores every output plane, releases the
 // slots, and advances the plane counter q. Returns false if the CTA aborts.
 template <class Cfg, int STEP, bool ENS, bool DTDEV, bool DIAG, class PT>
 __device__ __forceinline__ bool
 consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
-             long long lt, state_t* out, lo16_t* in_lo, lo16_t* out_lo, const void* ring,
+             const Piece& pc, state_t* out, lo16_t* in_lo, lo16_t* out_lo, const void* ring,
              uint64_t* full, uint64_t* empty, volatile int* abort_flag, uint32_t& q,
              const void* centre, uint64_t* full_c, uint64_t* empty_c, uint32_t& oq,
              DiagAcc& dacc)
@@ -1102,15 +1185,22 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
     const int tx   = tid % TX;
     const int ty   = tid / TX;
     const Layout& L = gv.L;
-    const TaskGeom<Cfg> tg(gv, lt, (long long)gv.ntx * gv.nty);
+    const TaskGeom<Cfg> tg(gv, pc);
     const int nload = tg.nout + 2 * NGHOST;
     const int i     = tg.i0 + tx;
     const int j     = tg.j0 + ty;
     const bool act  = (i >= gv.start.x) && (i < gv.end.x) && (j < gv.end.y);
     const T rkA     = a.P.rkA;
     T rkB           = a.P.rkB;
-    if constexpr (DTDEV)
+    if constexpr (DTDEV) {
         rkB = (T)(a.P.rk_beta * *a.P.dt_dev);
+        // formed here, not again at every plane
+#if AC_DOUBLE_PRECISION == 1
+        asm volatile("" : "+d"(rkB));
+#else
+        asm volatile("" : "+f"(rkB));
+#endif
+    }
     // this thread's column in a ring slot (elements)
     const int col = (ty + NGHOST) * BX + (tx + 4);
 
@@ -1365,11 +1455,9 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
 // slots, each guarded by a `full` barrier (transaction bytes) and an `empty`
 // barrier on which every consumer warp arrives once it has finished with the
 // plane. Consumer warps own one vertex column each and never wait for each
-// other except through the ring. Tasks (tile, z segment) are dealt round-robin
-// so the CTAs of one wave stream neighbouring tiles at the same z and their
-// halo reads of each other's planes hit L2. With ENS the tasks of all members
-// of an ensemble form one list (member-major) and each task reads its member's
-// map, geometry, buffers and parameters from the descriptor table.
+// other except through the ring. Which planes of which tiles a CTA marches:
+// Pieces. With ENS every piece names its member, whose map, geometry and buffers
+// are read from the descriptor table and whose parameters from the launch.
 template <bool ENS>
 using SolveKernelArgs = typename std::conditional<ENS, EnsSolveArgs<AcReal>, SolveArgs<AcReal>>::type;
 
@@ -1491,8 +1579,6 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     }
     __syncthreads();
 
-    const long long ntasks = ENS ? a.total_tasks : a.g.tasks; // (ENS: the group's tasks)
-
     if constexpr (Cfg::WGSPEC) {
         // whole warpgroups: warps 0..7 consume, warps 8..11 produce
         if (warp >= CWARPS)
@@ -1510,24 +1596,24 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
             uint32_t oq = 0; // output planes whose centre arrays were issued
             bool ok     = true;
             int last_m  = -1;
-            for (long long t = blockIdx.x; t < ntasks && ok; t += gridDim.x) {
+            PieceList<ENS> pieces(a);
+            while (ok) {
                 const CUtensorMap* map = &tin;
                 const SolveGeom* g     = &a.g;
-                long long lt           = t;
+                Piece pc;
+                if (!pieces.next(a, pc))
+                    break;
                 if constexpr (ENS) {
-                    const long long tg_      = t + a.task_base; // task in the whole list
-                    const int m              = member_of(a.members, a.nmembers, tg_);
-                    const MemberDesc<T>* md  = a.members + m;
-                    map                      = &md->tmap;
-                    g                        = &md->g;
-                    lt                       = tg_ - md->task_begin;
-                    if (m != last_m) {
+                    const MemberDesc<T>* md = a.members + pc.member;
+                    map                     = &md->tmap;
+                    g                       = &md->g;
+                    if (pc.member != last_m) {
                         fence_tensormap_acquire(map);
                         prefetch_tensormap(map);
-                        last_m = m;
+                        last_m = pc.member;
                     }
                 }
-                const TaskGeom<Cfg> tg(*g, lt, (long long)g->ntx * g->nty);
+                const TaskGeom<Cfg> tg(*g, pc);
                 const int xt    = g->L.offx + tg.i0 - 4; // a multiple of 16 bytes by construction
                 const int yt    = tg.j0 - NGHOST;
                 const int nload = tg.nout + 2 * NGHOST;
@@ -1593,22 +1679,21 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     uint32_t q = 0, oq = 0;
     DiagAcc dacc;
     diag_init(dacc);
-    for (long long t = blockIdx.x; t < ntasks; t += gridDim.x) {
+    PieceList<ENS> pieces(a);
+    Piece pc;
+    while (pieces.next(a, pc)) {
         bool ok;
         if constexpr (ENS) {
-            // the group's members: descriptor table and parameters from the
-            // launch (a.members points at the group's first descriptor)
-            const long long tg_     = t + a.task_base;
-            const int m             = member_of(a.members, a.nmembers, tg_);
-            const MemberDesc<T>* md = a.members + m;
+            // the member's descriptor, and its parameters from the launch
+            const MemberDesc<T>* md = a.members + pc.member;
             const SolveGeom gv      = md->g;
-            ok = consume_task<Cfg, STEP, ENS, DTDEV, false>(a, gv, a.mp[m], tg_ - md->task_begin,
-                                                     md->out, md->in_lo, md->out_lo, ring, full,
-                                                     empty, &abort_flag, q, centre, full_c,
-                                                     empty_c, oq, dacc);
+            ok = consume_task<Cfg, STEP, ENS, DTDEV, false>(a, gv, a.mp[pc.member], pc, md->out,
+                                                            md->in_lo, md->out_lo, ring, full,
+                                                            empty, &abort_flag, q, centre, full_c,
+                                                            empty_c, oq, dacc);
         }
         else {
-            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG>(a, a.g, a.P.rhs, t, a.out, a.in_lo, a.out_lo,
+            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG>(a, a.g, a.P.rhs, pc, a.out, a.in_lo, a.out_lo,
                                                     ring, full, empty, &abort_flag, q, centre,
                                                     full_c, empty_c, oq, dacc);
         }

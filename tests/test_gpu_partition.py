@@ -1,5 +1,6 @@
-"""The whole-box wall fill and the direct copies of a mesh that lies in GPU
-memory, at the sizes where each can go wrong."""
+"""The split of a launch's tile columns over the CTAs, the ghost images that a
+substep writes, the whole-box wall fill and the direct copies of a mesh that lies
+in GPU memory, at the sizes where each can go wrong."""
 import ctypes as C
 import math
 
@@ -15,6 +16,82 @@ FLAVOURS = ("sp", "dp", "mixed")
 def mesh_info(prec, n, **more):
     return abi.make_info(prec, *n, dsx=2 * math.pi / n[0], dsy=2 * math.pi / n[1],
                          dsz=2 * math.pi / n[2], gamma=5 / 3, nu_visc=5e-3, eta=5e-3, **more)
+
+
+# one plane a CTA; slabs and shares of what they leave; a share across two
+# columns; whole columns and a partial wave after them; the smallest mesh
+@pytest.mark.parametrize("n", [(3, 3, 3), (32, 30, 40), (97, 50, 75), (200, 190, 33),
+                               (420, 160, 9)])
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_every_plane_of_every_column_once(flavour, n):
+    """A step through each tile configuration (each splits the mesh differently)
+    equals the step taken as sub-boxes of two planes, bit for bit."""
+    prec = abi.PRECISIONS[flavour]
+    info = mesh_info(prec, n)
+    fields = init.workload_fields(*n, prec.np_dtype, seed=3, amplitude=1e-2, velocity_mode=0.1)
+    host = abi.HostMesh(prec, info, fields)
+    g, dt = abi.NGHOST, 1e-3
+
+    def stepped(dev, boxes):
+        dev.load_mesh(host)
+        for s in range(3):
+            dev.periodic_boundconds()
+            for lo, hi in boxes:
+                dev.integrate_substep(s, dt, lo, hi)
+            dev.swap_buffers()
+        out = abi.HostMesh(prec, info)
+        dev.store_mesh(out)
+        assert dev.status() == 0
+        return [out.interior(w).copy() for w in range(8)]
+
+    with Device(flavour, info) as dev:
+        slabs = [(abi.int3(g, g, g + z), abi.int3(g + n[0], g + n[1], g + min(z + 2, n[2])))
+                 for z in range(0, n[2], 2)]
+        want = stepped(dev, slabs)
+        for cfg in range(dev.solve_config()[1]):
+            dev.set_solve_config(cfg)
+            got = stepped(dev, [dev.interior_box()])
+            for w in range(8):
+                assert np.array_equal(got[w], want[w]), (cfg, w)
+
+
+# the smallest mesh that writes images (6 an axis), meshes below it, rows and
+# columns that end within a tile, every vertex near two faces, a long axis
+@pytest.mark.parametrize("n", [(6, 6, 6), (5, 9, 12), (7, 6, 11), (33, 13, 8), (40, 12, 50),
+                               (64, 64, 64), (200, 9, 7)])
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_whole_steps_equal_the_substep_loop(flavour, n):
+    """Whole steps, whose substeps write the ghost images on small meshes, leave
+    the very state, ghosts and lo parts included, that ghost fills, substeps and
+    buffer swaps leave."""
+    prec = abi.PRECISIONS[flavour]
+    info = mesh_info(prec, n)
+    fields = init.workload_fields(*n, prec.np_dtype, seed=4, amplitude=1e-2, velocity_mode=0.1)
+    host, dt = abi.HostMesh(prec, info, fields), 1e-3
+
+    def loop(dev):
+        for _ in range(3):
+            for s in range(3):
+                dev.periodic_boundconds()
+                dev.integrate_substep(s, dt)
+                dev.swap_buffers()
+
+    def steps(dev):
+        for _ in range(3):
+            dev.integrate_step(dt)
+
+    got = []
+    for advance in (loop, steps, lambda dev: dev.integrate_steps(dt, 3)):
+        with Device(flavour, info) as dev:
+            dev.load_mesh(host)
+            advance(dev)
+            got.append([dev.store_double(w) for w in range(8)])
+            dev.periodic_boundconds()
+            got[-1] += [dev.store_double(w) for w in range(8)]
+            assert dev.status() == 0
+    for other in got[1:]:
+        for w in range(16):
+            assert np.array_equal(got[0][w], other[w]), w
 
 
 @pytest.mark.parametrize("n", [(4, 4, 4), (8, 5, 6), (21, 9, 4), (124, 7, 5), (130, 4, 9)])
