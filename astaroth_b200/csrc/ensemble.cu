@@ -329,8 +329,8 @@ launch_halo_all(Ensemble e, cudaStream_t st)
     const int n          = (int)e->m.size();
     const long long want = (e->halo_total + 255) / 256;
     const int blocks     = (int)std::max<long long>(1, std::min<long long>(want, e->num_sms * 32));
-    halo_batch_kernel<<<blocks, 256, 0, st>>>(e->d_halo[e->cur], n, e->halo_total);
-    ACB_CUDA_CHECK(cudaGetLastError());
+    ACB_CUDA_CHECK(launch_overlapped(halo_batch_kernel, blocks, 256, 0, st,
+                                     (const HaloMember*)e->d_halo[e->cur], n, e->halo_total));
     e->launches++;
     e->ghost_ok[e->cur] = true;
     return AC_SUCCESS;
@@ -366,9 +366,8 @@ launch_solve_all(Ensemble e, cudaStream_t st, int step, AcReal dt)
             a.mp[i] = e->h_mp[g0 + i];
         const int grid = e->groups[g].grid;
         // the map parameter is not read in ensemble mode; any valid map fills it
-        ((EnsKernelFn)cfg.kern[step])<<<grid, cfg.threads, cfg.smem, st>>>(D[0].tmap, a,
-                                                                           no_centre_maps);
-        ACB_CUDA_CHECK(cudaGetLastError());
+        ACB_CUDA_CHECK(launch_overlapped((EnsKernelFn)cfg.kern[step], grid, cfg.threads, cfg.smem,
+                                         st, D[0].tmap, a, no_centre_maps));
         e->launches++;
     }
     e->ghost_ok[e->cur ^ 1] = false; // the out blocks' ghosts are stale now

@@ -30,6 +30,7 @@
 // box, lane-strided; kept for the reference's partial-box API calls.
 #pragma once
 #include "common.cuh"
+#include "tma.cuh"
 
 struct HaloArgs {
     Layout L;
@@ -269,6 +270,7 @@ halo_full_kernel(const Layout L, void* block, unsigned units_a, unsigned units, 
                  helem_t flip)
 {
     const unsigned stride = gridDim.x * blockDim.x;
+    grid_wait();
     for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < units; u += stride)
         halo_unit_block<MIRROR>(L, static_cast<helem_t*>(block), units_a, u, narr, flip);
 }
@@ -297,6 +299,7 @@ halo_batch_kernel(const HaloMember* __restrict__ mem, int n, long long total_uni
     for (int i = threadIdx.x; i < ns; i += blockDim.x)
         first[i] = mem[i].unit_begin;
     __syncthreads();
+    grid_wait(); // (the table itself is written by no kernel)
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < total_units;
          u += stride) {

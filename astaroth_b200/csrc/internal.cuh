@@ -5,6 +5,8 @@
 #pragma once
 #include <stdio.h>
 
+#include <utility>
+
 #include "astaroth.h"
 #include "common.cuh"
 #include "solve.cuh"
@@ -59,6 +61,10 @@ struct SolveConfig {
     // single mesh: substeps 0, 1, 2 reading the time step from device memory
     // (null in the ensemble table)
     const void* kern_dt[3];
+    // single mesh, substeps 0 and 1 also writing the periodic images of their
+    // output: time step given, and read from device memory (null in the ensemble
+    // table)
+    const void* kern_img[2][2];
     // single mesh, substep 2 also folding the step diagnostics of its output:
     // plain, with helical forcing, and reading the time step from device memory
     // (null in the ensemble table)
@@ -97,6 +103,7 @@ make_solve_config(double plane_cost)
     if constexpr (ENS) {
         c.kern[3]    = nullptr;
         c.kern_dt[0] = c.kern_dt[1] = c.kern_dt[2] = nullptr;
+        c.kern_img[0][0] = c.kern_img[0][1] = c.kern_img[1][0] = c.kern_img[1][1] = nullptr;
         c.kern_diag[0] = c.kern_diag[1] = c.kern_diag[2] = nullptr;
     }
     else {
@@ -104,6 +111,10 @@ make_solve_config(double plane_cost)
         c.kern_dt[0] = (const void*)solve_kernel<Cfg, 0, ENS, true>;
         c.kern_dt[1] = (const void*)solve_kernel<Cfg, 1, ENS, true>;
         c.kern_dt[2] = (const void*)solve_kernel<Cfg, 2, ENS, true>;
+        c.kern_img[0][0] = (const void*)solve_kernel<Cfg, 0, ENS, false, false, true>;
+        c.kern_img[0][1] = (const void*)solve_kernel<Cfg, 1, ENS, false, false, true>;
+        c.kern_img[1][0] = (const void*)solve_kernel<Cfg, 0, ENS, true, false, true>;
+        c.kern_img[1][1] = (const void*)solve_kernel<Cfg, 1, ENS, true, false, true>;
         c.kern_diag[0] = (const void*)solve_kernel<Cfg, 2, ENS, false, true>;
         c.kern_diag[1] = (const void*)solve_kernel<Cfg, 3, ENS, false, true>;
         c.kern_diag[2] = (const void*)solve_kernel<Cfg, 2, ENS, true, true>;
@@ -112,6 +123,27 @@ make_solve_config(double plane_cost)
 }
 
 namespace acb_host {
+
+// Launches a kernel that calls grid_wait (tma.cuh), so that its launch and set-up
+// run under the end of the kernel before it in the stream: 0.3 us a kernel (a 64^3
+// FP32 step of six 57.2 -> 55.3 us, 32^3 29.7 -> 28.7; nothing from 128^3 on).
+template <class... P, class... A>
+cudaError_t
+launch_overlapped(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                  cudaStream_t st, A&&... args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim            = dim3(grid);
+    c.blockDim           = dim3(block);
+    c.dynamicSmemBytes   = smem;
+    c.stream             = st;
+    c.attrs              = attr;
+    c.numAttrs           = 1;
+    return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
 
 constexpr int kDefaultSolveConfig = 0;
 

@@ -18,6 +18,7 @@
 // folds the partials in a fixed order (deterministic, no atomics on data).
 #pragma once
 #include "common.cuh"
+#include "tma.cuh"
 
 enum { RED_SCAL = 1, RED_VEC = 3, RED_ALFVEN = 4 };
 
@@ -280,6 +281,7 @@ reduce_sets_kernel(const ReduceArgs a)
         mn[t] = INFINITY;
         sm[t] = 0.0;
     }
+    grid_wait();
     red_rows<THREADS, NF>(
         a,
         [&](long long id, double* v) {

@@ -1164,10 +1164,48 @@ fence_tensormap_acquire(const CUtensorMap* map)
                  : "memory");
 }
 
+// Stores the periodic images of vertex (i, j, k), whose element in the first array
+// is id: the ghost vertices, up to one on each axis and their combinations, that a
+// fill of the out block would copy it to (n >= 6 on every axis). For meshes that
+// stay in L2, where it replaces the fill of the next substep (launch_solve); in a
+// large one the lone 32-byte sectors of the x ghosts cost DRAM more than the fill.
+template <class E, int N>
+__device__ __forceinline__ void
+store_images(const Layout& L, E* __restrict__ out, long long id, int i, int j, int k,
+             const E (&r)[N])
+{
+    const int dx = i < 2 * NGHOST ? L.nx : (i >= L.nx ? -L.nx : 0);
+    const int dy = j < 2 * NGHOST ? L.ny : (j >= L.ny ? -L.ny : 0);
+    const int dz = k < 2 * NGHOST ? L.nz : (k >= L.nz ? -L.nz : 0);
+    auto put = [&](long long d) {
+#pragma unroll
+        for (int a = 0; a < N; ++a)
+            out[a * L.fstride + id + d] = r[a];
+    };
+    const long long ey = (long long)dy * L.mxp, ez = (long long)dz * L.plane;
+    if (dx)
+        put(dx);
+    if (dy) {
+        put(ey);
+        if (dx)
+            put(ey + dx);
+    }
+    if (dz) {
+        put(ez);
+        if (dx)
+            put(ez + dx);
+        if (dy) {
+            put(ez + ey);
+            if (dx)
+                put(ez + ey + dx);
+        }
+    }
+}
+
 // One task of a consumer warp: the planes of one (tile, z segment) column.
 // Waits for the ring, computes and stores every output plane, releases the
 // slots, and advances the plane counter q. Returns false if the CTA aborts.
-template <class Cfg, int STEP, bool ENS, bool DTDEV, bool DIAG, class PT>
+template <class Cfg, int STEP, bool ENS, bool DTDEV, bool DIAG, bool IMAGES, class PT>
 __device__ __forceinline__ bool
 consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
              const Piece& pc, state_t* out, lo16_t* in_lo, lo16_t* out_lo, const void* ring,
@@ -1336,6 +1374,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                 // lane 0 of arrays 0..3 holds lnrho, ux, uy, uz: their stored
                 // values for the step diagnostics (hi and, mixed, lo)
                 float dh[ACB_NARR], dl[ACB_NARR];
+                acb::F2 res[ACB_NARR];
 #pragma unroll
                 for (int ar = 0; ar < ACB_NARR; ++ar) {
                     const int fa = acb_field(ar, 0), fb = acb_field(ar, 1);
@@ -1354,6 +1393,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     if (STEP == 3 && ar >= 1)
                         acb::pair_add2(h2, w2, acb::pk2(fo[ar - 1], 0.f), h2, w2);
                     o2[e] = h2;
+                    res[ar] = h2;
                     const uint32_t wl = lo_pack(w2); // lo rounded to bf16 as stored
                     if (ar & 1)
                         ol2[(ar >> 1) * L.fstride + id] =
@@ -1375,6 +1415,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     if (STEP == 3 && ar >= 1)
                         r = acb::add2(r, acb::pk2(fo[ar - 1], 0.f));
                     o2[e] = r;
+                    res[ar] = r;
                     if constexpr (DIAG) {
                         float t_;
                         acb::upk2(r, dh[ar], t_);
@@ -1382,6 +1423,8 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     }
 #endif
                 }
+                if constexpr (IMAGES)
+                    store_images(L, o2, id, i, j, k, res);
                 if constexpr (DIAG) {
                     // (double)hi + (double)lo, as the reductions read a value
                     double v[4];
@@ -1395,6 +1438,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     diag_add(dacc, v[0], v[1], v[2], v[3]);
                 }
                 (void)dh;
+                (void)res;
                 (void)dl;
             }
             else {
@@ -1411,7 +1455,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                                           [&] { load_centre<STEP>(L, out, id, cv); });
                 if constexpr (STEP == 3)
                     acb::forcing_at<T>(a.P, i, j, k, fo);
-                T dv[4];
+                T dv[4], res[ACB_NF];
 #pragma unroll
                 for (int f = 0; f < ACB_NF; ++f) {
                     T r;
@@ -1422,12 +1466,16 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
                     if (STEP == 3 && f >= 1 && f <= 3)
                         r += fo[f - 1];
                     out[fidx(L, f, id)] = r;
+                    res[f] = r;
                     if (f < 4)
                         dv[f] = r;
                 }
+                if constexpr (IMAGES)
+                    store_images(L, out, id, i, j, k, res);
                 if constexpr (DIAG)
                     diag_add(dacc, (double)dv[0], (double)dv[1], (double)dv[2], (double)dv[3]);
                 (void)dv;
+                (void)res;
             }
         }
         __syncwarp();
@@ -1535,9 +1583,13 @@ diag_finish(const SolveArgs<AcReal>& a, DiagAcc d)
 
 // DTDEV: the time step is read from device memory (SolveParams::dt_dev), for
 // steps whose time step the device chooses; single meshes, no forcing.
+// IMAGES: the launch also writes the periodic images of its output (single
+// meshes, the whole interior, n >= 6 on every axis); its code costs the plane loop
+// 3 % even where it is skipped, so the other kernels have none of it.
 // DIAG: the launch also folds the step diagnostics of its output (diag_finish);
 // single meshes, the last substep over the whole interior.
-template <class Cfg, int STEP, bool ENS, bool DTDEV = false, bool DIAG = false>
+template <class Cfg, int STEP, bool ENS, bool DTDEV = false, bool DIAG = false,
+          bool IMAGES = false>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     solve_kernel(const __grid_constant__ CUtensorMap tin,
                  const __grid_constant__ SolveKernelArgs<ENS> a,
@@ -1576,8 +1628,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
         }
         fence_barrier_init();
         abort_flag = 0;
+        if (!ENS)
+            prefetch_tensormap(&tin);
     }
     __syncthreads();
+    grid_wait();
 
     if constexpr (Cfg::WGSPEC) {
         // whole warpgroups: warps 0..7 consume, warps 8..11 produce
@@ -1590,8 +1645,6 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     if (warp >= CWARPS) {
         // ------------------------------------------------------------ producer
         if (warp == CWARPS && lane == 0) {
-            if (!ENS)
-                prefetch_tensormap(&tin);
             uint32_t q  = 0;
             uint32_t oq = 0; // output planes whose centre arrays were issued
             bool ok     = true;
@@ -1687,13 +1740,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
             // the member's descriptor, and its parameters from the launch
             const MemberDesc<T>* md = a.members + pc.member;
             const SolveGeom gv      = md->g;
-            ok = consume_task<Cfg, STEP, ENS, DTDEV, false>(a, gv, a.mp[pc.member], pc, md->out,
+            ok = consume_task<Cfg, STEP, ENS, DTDEV, false, false>(a, gv, a.mp[pc.member], pc, md->out,
                                                             md->in_lo, md->out_lo, ring, full,
                                                             empty, &abort_flag, q, centre, full_c,
                                                             empty_c, oq, dacc);
         }
         else {
-            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG>(a, a.g, a.P.rhs, pc, a.out, a.in_lo, a.out_lo,
+            ok = consume_task<Cfg, STEP, ENS, DTDEV, DIAG, IMAGES>(a, a.g, a.P.rhs, pc, a.out, a.in_lo, a.out_lo,
                                                     ring, full, empty, &abort_flag, q, centre,
                                                     full_c, empty_c, oq, dacc);
         }

@@ -114,3 +114,16 @@ prefetch_tensormap(const CUtensorMap* map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
+
+// Programmatic dependent launch: a kernel launched with the attribute is set up
+// while the last CTAs of the kernel before it in the stream still run. grid_wait()
+// returns once that kernel has finished and its writes are visible; every thread
+// calls it before it touches global memory, which also keeps the order transitive
+// (a kernel cannot finish before all earlier ones have). No kernel here releases
+// the next one early (griddepcontrol.launch_dependents): a solve CTA that waits
+// holds an SM that other streams' kernels, the awaited fill among them, could use.
+__device__ __forceinline__ void
+grid_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
