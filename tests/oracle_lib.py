@@ -192,7 +192,7 @@ def normwise_error(candidate: np.ndarray, model: np.ndarray) -> float:
 
 def cfl_dt(prec, info, umax: float, timescale: float = 1.0) -> float:
     """The Courant time step as the library evaluates it on the device
-    (astaroth_b200/csrc/device.cu: cfl_kernel): the reference standalone's
+    (astaroth_b200/csrc/reduce.cuh: cfl_step): the reference standalone's
     host_timestep (samples/standalone/model/host_timestep.cc:33-60, vAmax = 0)
     in double precision instead of long double, umax rounded to AcReal first,
     AC_dsmin or else the smallest spacing, the product with timescale in AcReal."""
