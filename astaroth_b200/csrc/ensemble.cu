@@ -205,7 +205,8 @@ schedule(const std::vector<Piece>& units, int slots, bool level,
 
 // (Re)builds both parities' descriptor tables and ghost-fill tables and the
 // schedule for the current tile configuration and segment length, and uploads
-// them.
+// them on the ensemble's stream: it does not wait for the legacy one, on which a
+// copy from pageable memory may return before it has landed.
 AcResult
 build_tables(Ensemble e)
 {
@@ -235,10 +236,12 @@ build_tables(Ensemble e)
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return zseg_of(e->m[a].L) > zseg_of(e->m[b].L);
     });
+    std::vector<HaloMember> halo[2];
     for (int p = 0; p < 2; ++p) {
         std::vector<MemberDesc<AcReal>>& D = e->h_desc[p];
         D.assign(n, MemberDesc<AcReal>());
-        std::vector<HaloMember> H(n);
+        std::vector<HaloMember>& H = halo[p];
+        H.resize(n);
         long long units = 0;
         for (int pos = 0; pos < n; ++pos) {
             const int i      = order[pos];
@@ -268,10 +271,10 @@ build_tables(Ensemble e)
             units += halo_units(L);
         }
         e->halo_total  = units;
-        ACB_CUDA_CHECK(cudaMemcpy(e->d_desc[p], D.data(), sizeof(MemberDesc<AcReal>) * n,
-                                  cudaMemcpyHostToDevice));
-        ACB_CUDA_CHECK(cudaMemcpy(e->d_halo[p], H.data(), sizeof(HaloMember) * n,
-                                  cudaMemcpyHostToDevice));
+        ACB_CUDA_CHECK(cudaMemcpyAsync(e->d_desc[p], D.data(), sizeof(MemberDesc<AcReal>) * n,
+                                       cudaMemcpyHostToDevice, e->stream));
+        ACB_CUDA_CHECK(cudaMemcpyAsync(e->d_halo[p], H.data(), sizeof(HaloMember) * n,
+                                       cudaMemcpyHostToDevice, e->stream));
     }
     // the schedule: all groups' pieces, then all groups' first ones
     std::vector<Piece> pieces;
@@ -310,10 +313,13 @@ build_tables(Ensemble e)
                               pieces.size() * sizeof(Piece) + first.size() * sizeof(int)));
     Piece* dp = (Piece*)e->d_schedule;
     int* df   = (int*)(dp + pieces.size());
-    ACB_CUDA_CHECK(cudaMemcpy(dp, pieces.data(), pieces.size() * sizeof(Piece),
-                              cudaMemcpyHostToDevice));
-    ACB_CUDA_CHECK(cudaMemcpy(df, first.data(), first.size() * sizeof(int),
-                              cudaMemcpyHostToDevice));
+    ACB_CUDA_CHECK(cudaMemcpyAsync(dp, pieces.data(), pieces.size() * sizeof(Piece),
+                                   cudaMemcpyHostToDevice, e->stream));
+    ACB_CUDA_CHECK(cudaMemcpyAsync(df, first.data(), first.size() * sizeof(int),
+                                   cudaMemcpyHostToDevice, e->stream));
+    // the kernels index by these tables: all of them in place (and the host's
+    // copies read) before anything can be launched
+    ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
     for (size_t g = 0; g < e->groups.size(); ++g) {
         e->groups[g].pieces = dp + piece_at[g];
         e->groups[g].first  = df + first_at[g];
@@ -464,7 +470,7 @@ acEnsembleCreate(const int device_id, const int num_members, const AcMeshInfo* c
     ACB_CUDA_CHECK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device_id));
     ACB_CUDA_CHECK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
     ACB_CUDA_CHECK(cudaMalloc((void**)&e->status, sizeof(unsigned)));
-    ACB_CUDA_CHECK(cudaMemset(e->status, 0, sizeof(unsigned)));
+    ACB_CUDA_CHECK(cudaMemsetAsync(e->status, 0, sizeof(unsigned), e->stream));
     e->m.resize(num_members);
     for (int i = 0; i < num_members; ++i) {
         Member& mb = e->m[i];
@@ -482,11 +488,11 @@ acEnsembleCreate(const int device_id, const int num_members, const AcMeshInfo* c
         const size_t bytes = block_bytes(mb.L);
         for (int b = 0; b < 2; ++b) {
             ACB_CUDA_CHECK(cudaMalloc((void**)&mb.blk[b], bytes));
-            ACB_CUDA_CHECK(cudaMemset(mb.blk[b], 0, bytes));
+            ACB_CUDA_CHECK(cudaMemsetAsync(mb.blk[b], 0, bytes, e->stream));
 #if ACB_MIXED
             const size_t lb = lo_block_bytes(mb.L);
             ACB_CUDA_CHECK(cudaMalloc((void**)&mb.lo[b], lb));
-            ACB_CUDA_CHECK(cudaMemset(mb.lo[b], 0, lb));
+            ACB_CUDA_CHECK(cudaMemsetAsync(mb.lo[b], 0, lb, e->stream));
 #endif
         }
     }

@@ -1,0 +1,194 @@
+/* A stand-in for the CUDA runtime, preloaded by tests of the library's host code
+ * (no GPU, no kernel runs). Device memory is host memory. It models what ordering
+ * tests need: a copy from pageable memory or a memset on one stream may still be
+ * pending when the call returns, so a launch on another (non-blocking) stream
+ * before a synchronisation is counted as unordered. */
+#include <cuda_runtime_api.h>
+#include <stdlib.h>
+#include <string.h>
+
+static cudaError_t last;
+static int live, mallocs_until_failure = -1, launches, unordered, instantiated;
+static char pending[64]; /* by stream number; 0: the legacy stream */
+static int streams;
+
+void fake_fail_malloc(int n) { mallocs_until_failure = n; } /* the n-th from now, 0 the next */
+int fake_live_allocations(void) { return live; }
+int fake_launches(void) { return launches; }
+int fake_unordered_launches(void) { return unordered; }
+int fake_graphs_instantiated(void) { return instantiated; }
+
+static int number(cudaStream_t s) { return (int)(size_t)s; }
+
+cudaError_t cudaGetLastError(void)
+{
+    cudaError_t e = last;
+    last          = cudaSuccess;
+    return e;
+}
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { (void)d; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d)
+{
+    (void)d;
+    *v = a == cudaDevAttrMultiProcessorCount ? 148 : 0;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDeviceProperties_v2(struct cudaDeviceProp* p, int d)
+{
+    (void)d;
+    memset(p, 0, sizeof(*p));
+    strcpy(p->name, "fake GPU");
+    p->multiProcessorCount = 148;
+    return cudaSuccess;
+}
+cudaError_t cudaMalloc(void** p, size_t n)
+{
+    if (mallocs_until_failure >= 0 && mallocs_until_failure-- == 0) {
+        *p = NULL;
+        return last = cudaErrorMemoryAllocation;
+    }
+    ++live;
+    *p = calloc(1, n ? n : 1);
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p)
+{
+    if (p)
+        --live;
+    free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void** p, size_t n) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaMemset(void* p, int v, size_t n)
+{
+    memset(p, v, n);
+    pending[0] = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s)
+{
+    memset(p, v, n);
+    pending[number(s)] = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind k)
+{
+    memcpy(d, s, n);
+    pending[0] = k == cudaMemcpyHostToDevice;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind k,
+                            cudaStream_t st)
+{
+    (void)k;
+    memcpy(d, s, n);
+    pending[number(st)] = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize(void) { memset(pending, 0, sizeof(pending)); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { pending[number(s)] = 0; return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f)
+{
+    (void)f;
+    *s = (cudaStream_t)(size_t)++streams;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) { (void)s; return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f)
+{
+    (void)s, (void)e, (void)f;
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)1; return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned f) { (void)f; return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { (void)e; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { (void)e, (void)s; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { (void)e; return cudaSuccess; }
+/* each interval is shorter than the one before it, so a tuner keeps its last candidate */
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b)
+{
+    static float t = 1e6f;
+    (void)a, (void)b;
+    *ms = t -= 1.0f;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v)
+{
+    (void)f, (void)a, (void)v;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes* a, const void* f)
+{
+    (void)f;
+    memset(a, 0, sizeof(*a));
+    a->numRegs = 255;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* f, int b, size_t s)
+{
+    (void)f, (void)b, (void)s;
+    *n = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int b,
+                                                                   size_t s, unsigned flags)
+{
+    (void)flags;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, f, b, s);
+}
+static int encode(void) { return 0; }
+cudaError_t cudaGetDriverEntryPoint(const char* name, void** fn, unsigned long long flags,
+                                    enum cudaDriverEntryPointQueryResult* q)
+{
+    (void)flags;
+    *fn = strcmp(name, "cuTensorMapEncodeTiled") == 0 ? (void*)encode : NULL;
+    *q  = *fn ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
+    return cudaSuccess;
+}
+static cudaError_t launch(cudaStream_t st)
+{
+    ++launches;
+    for (int s = 0; s < (int)sizeof(pending); ++s)
+        if (pending[s] && s != number(st)) {
+            ++unordered;
+            break;
+        }
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** args, size_t smem, cudaStream_t s)
+{
+    (void)f, (void)g, (void)b, (void)args, (void)smem;
+    return launch(s);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args)
+{
+    (void)f, (void)args;
+    return launch(c->stream);
+}
+cudaError_t cudaStreamBeginCapture(cudaStream_t s, enum cudaStreamCaptureMode m)
+{
+    (void)s, (void)m;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g)
+{
+    (void)s;
+    *g = (cudaGraph_t)1;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned long long f)
+{
+    (void)g, (void)f;
+    *e = (cudaGraphExec_t)(size_t)++instantiated;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) { (void)g; return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { (void)e; return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t s)
+{
+    (void)e, (void)s;
+    return cudaSuccess;
+}

@@ -1,0 +1,56 @@
+"""The host side of an ensemble (schedule, uploads, graphs, tuner) on a stand-in
+CUDA runtime (fake_cudart.c): no GPU, no kernel runs."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from astaroth_b200 import abi
+
+TESTS = os.path.dirname(os.path.abspath(__file__))
+FLAVOURS = ("sp", "dp", "mixed")
+
+PREAMBLE = """
+import ctypes, sys
+from astaroth_b200 import Ensemble, abi
+from astaroth_b200.device import AcError
+fake = ctypes.CDLL(None)
+flavour, cache = sys.argv[1], sys.argv[2]
+prec = abi.PRECISIONS[flavour]
+def ensemble(n=(40, 24, 32)):
+    return Ensemble(flavour, [abi.make_info(prec, n[0] + 8 * k, n[1], n[2]) for k in range(3)])
+"""
+
+
+@pytest.fixture(scope="module")
+def fake_runtime(tmp_path_factory):
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    lib = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", f"-I{cuda}/include",
+                    os.path.join(TESTS, "fake_cudart.c"), "-o", lib], check=True)
+    return lib
+
+
+def run(fake_runtime, tmp_path, flavour, body):
+    env = dict(os.environ, LD_PRELOAD=fake_runtime, PYTHONPATH=abi.REPO)
+    r = subprocess.run([sys.executable, "-c", PREAMBLE + textwrap.dedent(body), flavour,
+                        str(tmp_path / "tune.txt")], env=env, capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_tables_are_in_place_before_a_launch(fake_runtime, tmp_path, flavour):
+    """Nothing is launched on the ensemble's non-blocking stream while an upload
+    or a memset of another stream may still be pending."""
+    run(fake_runtime, tmp_path, flavour, """
+        e = ensemble()
+        e.integrate_step(1e-3)
+        e.set_schedule(1, 16)
+        e.integrate_step(1e-3)
+        e.auto_optimize(cache)
+        assert fake.fake_launches() > 12
+        assert fake.fake_unordered_launches() == 0
+    """)
