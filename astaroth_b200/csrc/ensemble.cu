@@ -94,17 +94,16 @@ struct ensemble_s {
     int cur; // buffer parity: blk[cur] is `in` for every member
     int cfg;
     int seg_planes; // target planes per z segment (0: whole columns)
-    bool seg_given; // set by the caller or the tuner (else whole columns)
     // ghost_ok[p]: the ghosts of every member's block p hold periodic images
     bool ghost_ok[2];
     StageBuf stage; // staging buffer of member loads
 
-    bool desc_valid;
     std::vector<MemberDesc<AcReal>> h_desc[2];
     std::vector<RhsParams<AcReal>> h_mp; // by task-list position (both parities)
     // launch arguments of one group of members (about 20 KB, kept off the
     // stack; the launch copies them)
     std::unique_ptr<EnsSolveArgs<AcReal>> args;
+    void* d_tables; // the allocation that holds the tables below and the schedule
     MemberDesc<AcReal>* d_desc[2];
     HaloMember* d_halo[2];
     long long halo_total; // work units of one batched ghost fill
@@ -116,7 +115,6 @@ struct ensemble_s {
         int* first;
     };
     std::vector<Group> groups;
-    void* d_schedule; // one allocation for all groups
 
     unsigned long long launches;
     unsigned long long version; // bumped on any schedule change
@@ -203,25 +201,24 @@ schedule(const std::vector<Piece>& units, int slots, bool level,
         cta[c].insert(cta[c].end(), tail[c].begin(), tail[c].end());
 }
 
-// (Re)builds both parities' descriptor tables and ghost-fill tables and the
-// schedule for the current tile configuration and segment length, and uploads
-// them on the ensemble's stream: it does not wait for the legacy one, on which a
-// copy from pageable memory may return before it has landed.
+// Builds both parities' descriptor and ghost-fill tables and the schedule of a
+// tile configuration and segment length, and puts them in place of the ones in
+// use, which stay as they are if anything fails. They go up on the ensemble's
+// stream: it does not wait for the legacy one, on which a copy from pageable
+// memory may return before it has landed.
 AcResult
-build_tables(Ensemble e)
+build_tables(Ensemble e, int config, int seg_planes)
 {
     int ncfg;
     const SolveConfig* cfgs = ensemble_configs(&ncfg);
     if (prepare_table(cfgs, ncfg) != AC_SUCCESS)
         return AC_FAILURE;
-    const SolveConfig& cfg = cfgs[e->cfg];
+    const SolveConfig& cfg = cfgs[config];
     const int n            = (int)e->m.size();
     int per_sm             = 0;
     ACB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg.kern[1], cfg.threads,
                                                                  cfg.smem));
     per_sm = std::max(per_sm, 1);
-    e->h_mp.assign(n, RhsParams<AcReal>());
-    const int seg_planes = e->seg_given ? e->seg_planes : 0;
     // planes per unit of a member: its z range in equal segments
     auto zseg_of = [&](const Layout& L) {
         int nseg = 1;
@@ -236,22 +233,23 @@ build_tables(Ensemble e)
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return zseg_of(e->m[a].L) > zseg_of(e->m[b].L);
     });
+    std::vector<MemberDesc<AcReal>> desc[2];
     std::vector<HaloMember> halo[2];
+    std::vector<RhsParams<AcReal>> params(n);
+    long long halo_total = 0;
     for (int p = 0; p < 2; ++p) {
-        std::vector<MemberDesc<AcReal>>& D = e->h_desc[p];
-        D.assign(n, MemberDesc<AcReal>());
-        std::vector<HaloMember>& H = halo[p];
-        H.resize(n);
+        desc[p].assign(n, MemberDesc<AcReal>());
+        halo[p].resize(n);
         long long units = 0;
         for (int pos = 0; pos < n; ++pos) {
             const int i      = order[pos];
             const Member& mb = e->m[i];
             const Layout& L  = mb.L;
-            MemberDesc<AcReal>& d = D[pos];
-            memset(&d, 0, sizeof(d));
+            MemberDesc<AcReal>& d = desc[p][pos];
             if (encode_block_map(L, mb.blk[p], cfg, &d.tmap) != AC_SUCCESS)
                 return AC_FAILURE;
             SolveGeom& g = d.g;
+            memset(&g, 0, sizeof(g));
             g.L          = L;
             g.start      = make_int3(NGHOST, NGHOST, NGHOST);
             g.end        = make_int3(NGHOST + L.nx, NGHOST + L.ny, NGHOST + L.nz);
@@ -263,28 +261,25 @@ build_tables(Ensemble e)
             d.in_lo       = mb.lo[p];
             d.out_lo      = mb.lo[p ^ 1];
             if (p == 0)
-                e->h_mp[pos] = make_params(mb.uniforms, L, 0, 0).rhs;
-            H[pos].L          = L;
-            H[pos].block      = mb.blk[p];
-            H[pos].unit_begin = units;
-            H[pos].units_a    = (unsigned)halo_units_a(L);
+                params[pos] = make_params(mb.uniforms, L, 0, 0).rhs;
+            HaloMember& h = halo[p][pos];
+            h.L           = L;
+            h.block       = mb.blk[p];
+            h.unit_begin  = units;
+            h.units_a     = (unsigned)halo_units_a(L);
             units += halo_units(L);
         }
-        e->halo_total  = units;
-        ACB_CUDA_CHECK(cudaMemcpyAsync(e->d_desc[p], D.data(), sizeof(MemberDesc<AcReal>) * n,
-                                       cudaMemcpyHostToDevice, e->stream));
-        ACB_CUDA_CHECK(cudaMemcpyAsync(e->d_halo[p], H.data(), sizeof(HaloMember) * n,
-                                       cudaMemcpyHostToDevice, e->stream));
+        halo_total = units;
     }
     // the schedule: all groups' pieces, then all groups' first ones
     std::vector<Piece> pieces;
     std::vector<int> first;
     std::vector<size_t> piece_at, first_at;
-    e->groups.clear();
+    std::vector<ensemble_s::Group> groups;
     for (int g0 = 0; g0 < n; g0 += ACB_ENS_GROUP) {
         std::vector<Piece> units;
         for (int pos = g0; pos < std::min(n, g0 + ACB_ENS_GROUP); ++pos) {
-            const SolveGeom& g = e->h_desc[0][pos].g;
+            const SolveGeom& g = desc[0][pos].g;
             const int zseg     = zseg_of(g.L);
             for (int z0 = 0; z0 < g.nzr; z0 += zseg)
                 for (int t = 0; t < g.ntx * g.nty; ++t)
@@ -304,27 +299,59 @@ build_tables(Ensemble e)
             ++grid;
         }
         first.push_back(at);
-        e->groups.push_back({grid, nullptr, nullptr});
+        groups.push_back({grid, nullptr, nullptr});
     }
-    if (e->d_schedule)
-        cudaFree(e->d_schedule);
-    e->d_schedule = nullptr;
-    ACB_CUDA_CHECK(cudaMalloc(&e->d_schedule,
-                              pieces.size() * sizeof(Piece) + first.size() * sizeof(int)));
-    Piece* dp = (Piece*)e->d_schedule;
-    int* df   = (int*)(dp + pieces.size());
-    ACB_CUDA_CHECK(cudaMemcpyAsync(dp, pieces.data(), pieces.size() * sizeof(Piece),
-                                   cudaMemcpyHostToDevice, e->stream));
-    ACB_CUDA_CHECK(cudaMemcpyAsync(df, first.data(), first.size() * sizeof(int),
-                                   cudaMemcpyHostToDevice, e->stream));
-    // the kernels index by these tables: all of them in place (and the host's
-    // copies read) before anything can be launched
-    ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    for (size_t g = 0; g < e->groups.size(); ++g) {
-        e->groups[g].pieces = dp + piece_at[g];
-        e->groups[g].first  = df + first_at[g];
+    // one allocation for all of them, each table aligned as the allocation is
+    struct Part {
+        const void* from;
+        size_t bytes, at;
+    };
+    Part part[] = {{desc[0].data(), sizeof(desc[0][0]) * n, 0},
+                   {desc[1].data(), sizeof(desc[1][0]) * n, 0},
+                   {halo[0].data(), sizeof(halo[0][0]) * n, 0},
+                   {halo[1].data(), sizeof(halo[1][0]) * n, 0},
+                   {pieces.data(), sizeof(Piece) * pieces.size(), 0},
+                   {first.data(), sizeof(int) * first.size(), 0}};
+    size_t total = 0;
+    for (Part& q : part) {
+        q.at = total;
+        total += (q.bytes + 255) / 256 * 256;
     }
-    e->desc_valid = true;
+    char* tables = nullptr;
+    cudaError_t err = cudaMalloc((void**)&tables, total);
+    for (const Part& q : part)
+        if (err == cudaSuccess)
+            err = cudaMemcpyAsync(tables + q.at, q.from, q.bytes, cudaMemcpyHostToDevice,
+                                  e->stream);
+    // the kernels index by these tables: all of them in place (the host's copies
+    // read, and the tables in use read for the last time) before they are used
+    if (err == cudaSuccess)
+        err = cudaStreamSynchronize(e->stream);
+    if (err != cudaSuccess) {
+        fprintf(stderr, "astaroth_b200: ensemble tables (%zu bytes): %s\n", total,
+                cudaGetErrorString(err));
+        cudaGetLastError(); // reported here, not to the next check
+        if (tables)
+            cudaFree(tables);
+        return AC_FAILURE;
+    }
+    if (e->d_tables)
+        cudaFree(e->d_tables);
+    e->d_tables = tables;
+    for (int p = 0; p < 2; ++p) {
+        e->h_desc[p].swap(desc[p]);
+        e->d_desc[p] = (MemberDesc<AcReal>*)(tables + part[p].at);
+        e->d_halo[p] = (HaloMember*)(tables + part[2 + p].at);
+    }
+    for (size_t g = 0; g < groups.size(); ++g) {
+        groups[g].pieces = (Piece*)(tables + part[4].at) + piece_at[g];
+        groups[g].first  = (int*)(tables + part[5].at) + first_at[g];
+    }
+    e->groups.swap(groups);
+    e->h_mp.swap(params);
+    e->halo_total = halo_total;
+    e->cfg        = config;
+    e->version++;
     drop_graphs(e);
     return AC_SUCCESS;
 }
@@ -465,7 +492,6 @@ acEnsembleCreate(const int device_id, const int num_members, const AcMeshInfo* c
     ACB_CUDA_CHECK(cudaSetDevice(device_id));
     Ensemble e = new ensemble_s();
     e->id      = device_id;
-    e->cfg     = kDefaultSolveConfig;
     e->seg_planes = 32;
     ACB_CUDA_CHECK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device_id));
     ACB_CUDA_CHECK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
@@ -503,11 +529,7 @@ acEnsembleCreate(const int device_id, const int num_members, const AcMeshInfo* c
         acEnsembleDestroy(e);
         return AC_FAILURE;
     }
-    for (int p = 0; p < 2; ++p) {
-        ACB_CUDA_CHECK(cudaMalloc((void**)&e->d_desc[p], sizeof(MemberDesc<AcReal>) * num_members));
-        ACB_CUDA_CHECK(cudaMalloc((void**)&e->d_halo[p], sizeof(HaloMember) * num_members));
-    }
-    if (build_tables(e) != AC_SUCCESS) {
+    if (build_tables(e, kDefaultSolveConfig, 0) != AC_SUCCESS) {
         acEnsembleDestroy(e);
         return AC_FAILURE;
     }
@@ -530,14 +552,8 @@ acEnsembleDestroy(Ensemble e)
             if (mb.lo[b])
                 cudaFree(mb.lo[b]);
         }
-    for (int p = 0; p < 2; ++p) {
-        if (e->d_desc[p])
-            cudaFree(e->d_desc[p]);
-        if (e->d_halo[p])
-            cudaFree(e->d_halo[p]);
-    }
-    if (e->d_schedule)
-        cudaFree(e->d_schedule);
+    if (e->d_tables)
+        cudaFree(e->d_tables);
     if (e->status)
         cudaFree(e->status);
     stage_destroy(&e->stage);
@@ -676,12 +692,10 @@ acEnsembleSetSchedule(Ensemble e, const int config, const int segment_planes)
     if (config < 0 || config >= n || segment_planes < 0)
         return AC_FAILURE;
     cudaSetDevice(e->id);
-    ACB_CUDA_CHECK(cudaStreamSynchronize(e->stream));
-    e->cfg        = config;
+    if (build_tables(e, config, segment_planes) != AC_SUCCESS)
+        return AC_FAILURE;
     e->seg_planes = segment_planes;
-    e->seg_given  = true;
-    e->version++;
-    return build_tables(e);
+    return AC_SUCCESS;
 }
 
 AcResult

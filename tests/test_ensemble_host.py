@@ -54,3 +54,29 @@ def test_tables_are_in_place_before_a_launch(fake_runtime, tmp_path, flavour):
         assert fake.fake_launches() > 12
         assert fake.fake_unordered_launches() == 0
     """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_a_refused_schedule_leaves_the_one_in_use(fake_runtime, tmp_path, flavour):
+    """A schedule whose tables cannot be allocated is refused; the ensemble keeps
+    its tables, its schedule and its graphs, and goes on."""
+    run(fake_runtime, tmp_path, flavour, """
+        e = ensemble()
+        e.set_schedule(1, 16)
+        e.integrate_steps(1e-3, 2)
+        live, graphs = fake.fake_live_allocations(), fake.fake_graphs_instantiated()
+        fake.fake_fail_malloc(0)
+        try:
+            e.set_schedule(2, 8)
+            sys.exit("accepted")
+        except AcError:
+            pass
+        assert fake.fake_live_allocations() == live
+        assert e.schedule() == (1, 16)
+        e.integrate_steps(1e-3, 2)
+        assert fake.fake_graphs_instantiated() == graphs
+        e.set_schedule(2, 8)
+        assert e.schedule() == (2, 8) and fake.fake_live_allocations() == live
+        e.destroy()
+        assert fake.fake_live_allocations() == 0
+    """)
