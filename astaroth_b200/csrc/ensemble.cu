@@ -120,7 +120,7 @@ struct ensemble_s {
     unsigned long long version; // bumped on any schedule change
     cudaGraphExec_t graph[2];
     unsigned long long graph_key[2];
-    float graph_dt[2];
+    AcReal graph_dt[2]; // the time step the graph was captured with, which it holds
     unsigned long long graph_launches[2];
     bool graph_ghost[2][2]; // ghost_ok of both blocks after a replay of graph[p]
 };
@@ -621,7 +621,7 @@ acEnsembleIntegrateSteps(Ensemble e, const AcReal dt, const int num_steps)
         const int p = e->cur;
         // a captured step contains the ghost fill only when the ghosts were stale
         const unsigned long long key = (e->version << 2) | (e->ghost_ok[p] ? 2ull : 0ull) | 1ull;
-        if (!e->graph[p] || e->graph_key[p] != key || e->graph_dt[p] != (float)dt) {
+        if (!e->graph[p] || e->graph_key[p] != key || e->graph_dt[p] != dt) {
             if (e->graph[p])
                 cudaGraphExecDestroy(e->graph[p]);
             e->graph[p] = nullptr;
@@ -642,7 +642,7 @@ acEnsembleIntegrateSteps(Ensemble e, const AcReal dt, const int num_steps)
             ACB_CUDA_CHECK(cudaGraphInstantiate(&e->graph[p], g, 0));
             cudaGraphDestroy(g);
             e->graph_key[p] = key;
-            e->graph_dt[p]  = (float)dt;
+            e->graph_dt[p]  = dt;
         }
         ACB_CUDA_CHECK(cudaGraphLaunch(e->graph[p], e->stream));
         e->launches += e->graph_launches[p];

@@ -80,3 +80,19 @@ def test_a_refused_schedule_leaves_the_one_in_use(fake_runtime, tmp_path, flavou
         e.destroy()
         assert fake.fake_live_allocations() == 0
     """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_a_graph_is_replayed_for_its_own_time_step_only(fake_runtime, tmp_path, flavour):
+    """A captured step holds its time step: the next value of the library's
+    precision takes a graph of its own (one for each buffer parity)."""
+    run(fake_runtime, tmp_path, flavour, """
+        import numpy as np
+        e, dt = ensemble(), prec.np_dtype(1e-3)
+        e.integrate_steps(dt, 6)  # both parities
+        graphs = fake.fake_graphs_instantiated()
+        e.integrate_steps(dt, 4)
+        assert fake.fake_graphs_instantiated() == graphs
+        e.integrate_steps(np.nextafter(dt, prec.np_dtype(1)), 2)
+        assert fake.fake_graphs_instantiated() == graphs + 2
+    """)
