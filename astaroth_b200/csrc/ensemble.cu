@@ -492,7 +492,6 @@ acEnsembleCreate(const int device_id, const int num_members, const AcMeshInfo* c
     ACB_CUDA_CHECK(cudaSetDevice(device_id));
     Ensemble e = new ensemble_s();
     e->id      = device_id;
-    e->seg_planes = 32;
     ACB_CUDA_CHECK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device_id));
     ACB_CUDA_CHECK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
     ACB_CUDA_CHECK(cudaMalloc((void**)&e->status, sizeof(unsigned)));

@@ -96,3 +96,11 @@ def test_a_graph_is_replayed_for_its_own_time_step_only(fake_runtime, tmp_path, 
         e.integrate_steps(np.nextafter(dt, prec.np_dtype(1)), 2)
         assert fake.fake_graphs_instantiated() == graphs + 2
     """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_a_new_ensemble_reports_the_schedule_it_runs(fake_runtime, tmp_path, flavour):
+    """Whole columns of the first configuration."""
+    run(fake_runtime, tmp_path, flavour, """
+        assert ensemble().schedule() == (0, 0)
+    """)
