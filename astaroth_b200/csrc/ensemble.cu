@@ -420,10 +420,24 @@ enqueue_step(Ensemble e, cudaStream_t st, AcReal dt)
     return AC_SUCCESS;
 }
 
+// What a cached choice was timed for: the GPU, the compiled tiles that its index
+// counts, how segment lengths are dealt (raised when schedule() changes), and
+// the members. One word: the cache file separates by blanks.
+constexpr int kScheduleVersion = 2;
+
 std::string
 cache_key(Ensemble e)
 {
     std::string k = ACB_MIXED ? "mixed" : (sizeof(AcReal) == 8 ? "dp" : "sp");
+    cudaDeviceProp prop;
+    if (cudaGetDeviceProperties(&prop, e->id) == cudaSuccess)
+        k += "|" + std::string(prop.name);
+    std::replace(k.begin(), k.end(), ' ', '_');
+    k += "|" + std::to_string(e->num_sms) + "|v" + std::to_string(kScheduleVersion);
+    int ncfg;
+    const SolveConfig* cfgs = ensemble_configs(&ncfg);
+    for (int c = 0; c < ncfg; ++c)
+        k += (c ? "," : "|") + std::string(cfgs[c].name);
     std::vector<std::string> dims;
     for (const Member& mb : e->m)
         dims.push_back(std::to_string(mb.L.nx) + "x" + std::to_string(mb.L.ny) + "x" +

@@ -179,9 +179,9 @@ AcResult acEnsembleGetLaunchCount(Ensemble ensemble, unsigned long long* count);
 AcResult acEnsembleSetSchedule(Ensemble ensemble, const int config, const int segment_planes);
 AcResult acEnsembleGetSchedule(Ensemble ensemble, int* config, int* segment_planes);
 /* Times every (configuration, segment length) pair on this ensemble and keeps
- * the fastest; results are cached in a text file keyed by the precision and
- * the member sizes (cache_path NULL: $ACB_TUNE_CACHE, else
- * ~/.cache/astaroth_b200/tune.txt). Only the scratch `out` buffers are
+ * the fastest; results are cached in a text file keyed by the precision, the
+ * GPU, the compiled configurations and the member sizes (cache_path NULL:
+ * $ACB_TUNE_CACHE, else ~/.cache/astaroth_b200/tune.txt). Only the scratch `out` buffers are
  * touched, so the members' states are preserved between whole steps. */
 AcResult acEnsembleAutoOptimize(Ensemble ensemble, const char* cache_path);
 

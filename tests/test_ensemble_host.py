@@ -104,3 +104,22 @@ def test_a_new_ensemble_reports_the_schedule_it_runs(fake_runtime, tmp_path, fla
     run(fake_runtime, tmp_path, flavour, """
         assert ensemble().schedule() == (0, 0)
     """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_a_choice_timed_on_other_kernels_is_not_taken(fake_runtime, tmp_path, flavour):
+    """The tuner's cache: an entry that names only the precision and the sizes, as
+    older ones do, misses; the entry of this library hits."""
+    run(fake_runtime, tmp_path, flavour, """
+        old = flavour + "|1*40x24x32|1*48x24x32|1*56x24x32 1 64\\n"
+        open(cache, "w").write(old)
+        e = ensemble()
+        e.auto_optimize(cache)
+        assert e.schedule() == (2, 16)  # the last one timed (see cudaEventElapsedTime)
+        text = open(cache).read()
+        assert text.startswith(old) and len(text.split()) == 6
+        launches = fake.fake_launches()
+        other = ensemble()
+        other.auto_optimize(cache)
+        assert other.schedule() == (2, 16) and fake.fake_launches() == launches
+    """)
