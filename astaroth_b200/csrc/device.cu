@@ -950,38 +950,50 @@ flat_mesh_kernel(const Layout L, state_t* __restrict__ block, lo16_t* __restrict
 }
 
 typedef CUresult (*PFN_pointerGetAttributes_t)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+typedef CUresult (*PFN_memGetAddressRange_t)(CUdeviceptr*, size_t*, CUdeviceptr);
+
+static void*
+driver_function(const char* name)
+{
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        fn = nullptr;
+    return fn;
+}
 
 // Whether n values from p on lie in one allocation of the current GPU, aligned
 // as values are, so that a kernel can read and write them in place. What does
-// not (host or managed memory, another GPU's, a range that no allocation holds)
-// goes through the staging buffer, whose copies refuse what cannot be copied.
+// not (host or managed memory, another GPU's, a range that no allocation holds,
+// virtual memory that the program maps itself, parts of which may be unmapped or
+// closed to this GPU) goes through the staging buffer, whose copies refuse what
+// cannot be copied.
 static bool
 on_this_gpu(const AcReal* p, size_t n)
 {
-    static const PFN_pointerGetAttributes_t get = [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            fn = nullptr;
-        return (PFN_pointerGetAttributes_t)fn;
-    }();
+    static const auto attributes =
+        (PFN_pointerGetAttributes_t)driver_function("cuPointerGetAttributes");
+    static const auto range = (PFN_memGetAddressRange_t)driver_function("cuMemGetAddressRange");
     unsigned type = 0, managed = 1; // as the driver leaves them for other pointers
     int dev = -1, ordinal = -2;
-    CUdeviceptr start = 0;
-    size_t size       = 0;
+    unsigned plain          = 0;       // cudaMalloc's, not mapped address space
+    CUmemoryPool pool       = nullptr; // cudaMallocAsync's
+    CUdeviceptr start       = 0;
+    size_t size             = 0;
+    const CUdeviceptr first = (CUdeviceptr)(uintptr_t)p;
     CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
                                   CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
-                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
-                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void* to[] = {&type, &managed, &ordinal, &start, &size};
-    if (!get || (uintptr_t)p % sizeof(AcReal) != 0 || cudaGetDevice(&dev) != cudaSuccess ||
-        get(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS)
+                                  CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE,
+                                  CU_POINTER_ATTRIBUTE_MEMPOOL_HANDLE};
+    void* to[] = {&type, &managed, &ordinal, &plain, &pool};
+    if (!attributes || !range || (uintptr_t)p % sizeof(AcReal) != 0 ||
+        cudaGetDevice(&dev) != cudaSuccess || attributes(5, what, to, first) != CUDA_SUCCESS ||
+        type != CU_MEMORYTYPE_DEVICE || managed || ordinal != dev || !(plain || pool) ||
+        range(&start, &size, first) != CUDA_SUCCESS)
         return false;
-    const size_t at = (size_t)((CUdeviceptr)(uintptr_t)p - start);
-    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == dev && at <= size &&
-           n <= (size - at) / sizeof(AcReal);
+    const size_t at = (size_t)(first - start);
+    return at <= size && n <= (size - at) / sizeof(AcReal);
 }
 
 AcResult

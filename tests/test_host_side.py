@@ -1,5 +1,6 @@
-"""The host side of an ensemble (schedule, uploads, graphs, tuner) on a stand-in
-CUDA runtime (fake_cudart.c): no GPU, no kernel runs."""
+"""The library's host code (an ensemble's schedule, uploads, graphs and tuner; the
+route of a mesh transfer) on a stand-in CUDA runtime (fake_cudart.c): no GPU, no
+kernel runs."""
 import os
 import subprocess
 import sys
@@ -122,4 +123,45 @@ def test_a_choice_timed_on_other_kernels_is_not_taken(fake_runtime, tmp_path, fl
         other = ensemble()
         other.auto_optimize(cache)
         assert other.schedule() == (2, 16) and fake.fake_launches() == launches
+    """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_a_mesh_that_is_not_all_mapped_is_refused(fake_runtime, tmp_path, flavour):
+    """A mesh in address space that the program maps itself is copied, not read and
+    written in place by a kernel: the driver reports the whole reservation as the
+    pointer's range, and only a copy refuses what is not mapped of it."""
+    run(fake_runtime, tmp_path, flavour, """
+        from astaroth_b200 import Device
+        n = (40, 24, 32)
+        info = abi.make_info(prec, *n)
+        cells = (n[0] + 6) * (n[1] + 6) * (n[2] + 6)
+        field = cells * ctypes.sizeof(prec.real)
+        host = (ctypes.c_char * (9 * field))()
+        base = ctypes.addressof(host)
+
+        def mesh(at):
+            m = abi.mesh_type(prec)()
+            m.info = info
+            for w in range(8):
+                m.vertex_buffer[w] = ctypes.cast(at + w * field, ctypes.POINTER(prec.real))
+            return m
+
+        def load_and_store(dev, m):
+            before = fake.fake_launches()
+            rc = (dev.lib.acDeviceLoadMesh(dev.handle, 0, m),
+                  dev.lib.acDeviceStoreMesh(dev.handle, 0, ctypes.byref(m)))
+            return rc, fake.fake_launches() - before
+
+        dev = Device(flavour, info)
+        plain = ctypes.c_void_p()
+        fake.cudaMalloc(ctypes.byref(plain), ctypes.c_size_t(8 * field))
+        assert load_and_store(dev, mesh(plain.value)) == ((0, 0), 2)
+        # all of it mapped: a copy and a kernel for each field
+        fake.fake_reserve(ctypes.c_void_p(base), ctypes.c_size_t(9 * field), ctypes.c_size_t(8 * field))
+        assert load_and_store(dev, mesh(base)) == ((0, 0), 16)
+        # the last field not
+        fake.fake_reserve(ctypes.c_void_p(base), ctypes.c_size_t(9 * field), ctypes.c_size_t(8 * field - 4))
+        rc, launches = load_and_store(dev, mesh(base))
+        assert rc == (1, 1) and launches > 2
     """)
