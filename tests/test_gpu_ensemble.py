@@ -141,3 +141,45 @@ def test_ensemble_larger_than_one_launch_group():
             dev.store_mesh(host)
         for w in range(8):
             assert np.array_equal(got[k][w], host.fields[w]), (k, w)
+
+
+@pytest.mark.parametrize("flavour", ["sp", "dp", "mixed"])
+def test_ensemble_of_several_rounds_of_columns(flavour):
+    """More columns than one round of CTAs: full rounds dealt one column each, and a
+    partial round whose columns are cut and levelled over all CTAs. Every member
+    equals its mesh advanced alone, bit for bit."""
+    import re
+
+    import torch
+
+    prec = abi.PRECISIONS[flavour]
+    sizes = [(96 + 32 * (k % 2), 50 + k, 20 + 7 * (k % 4)) for k in range(24)]
+    infos = [member_info(prec, n, k) for k, n in enumerate(sizes)]
+    hosts = [abi.HostMesh(prec, infos[k], member_fields(prec, n, k)) for k, n in enumerate(sizes)]
+    with Ensemble(flavour, infos) as ens:
+        # whole columns of the first configuration, one CTA for each SM
+        assert ens.schedule() == (0, 0)
+        tile = re.match(r"tile(\d+)x(\d+)_", ens.lib.acSolveConfigName(0).decode())
+        tx, ty = int(tile[1]), int(tile[2])
+        columns = sum(-(-nx // tx) * -(-ny // ty) for nx, ny, _ in sizes)
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert columns > sms and columns % sms != 0
+        for k, host in enumerate(hosts):
+            ens.load_member(k, host)
+        ens.integrate_step(1e-3)
+        ens.integrate_steps(1e-3, 2)
+        ens.synchronize()
+        assert ens.status() == 0
+        got = []
+        for k in range(len(sizes)):
+            h = abi.HostMesh(prec, infos[k])
+            ens.store_member(k, h)
+            got.append(h)
+    for k in range(len(sizes)):
+        with Device(flavour, infos[k]) as dev:
+            dev.load_mesh(hosts[k])
+            for _ in range(3):
+                dev.integrate_step(1e-3)
+            dev.store_mesh(hosts[k])
+        for w in range(8):
+            assert np.array_equal(got[k].interior(w), hosts[k].interior(w)), (k, w)

@@ -18,10 +18,15 @@ def mesh_info(prec, n, **more):
                          dsz=2 * math.pi / n[2], gamma=5 / 3, nu_visc=5e-3, eta=5e-3, **more)
 
 
-# one plane a CTA; slabs and shares of what they leave; a share across two
-# columns; whole columns and a partial wave after them; the smallest mesh
-@pytest.mark.parametrize("n", [(3, 3, 3), (32, 30, 40), (97, 50, 75), (200, 190, 33),
-                               (420, 160, 9)])
+# the smallest mesh; slabs of few planes; slabs and shares of what they leave, some
+# across two columns and more; z segments; whole columns, alone and with a partial
+# wave after them. Each library takes each of these forms at one of the sizes on a
+# GPU of 148 SMs: test_host_side.py (test_the_split_takes_every_form).
+SPLIT_SIZES = [(3, 3, 3), (32, 30, 40), (97, 50, 75), (200, 190, 33), (420, 160, 9),
+               (200, 168, 48), (200, 108, 48), (64, 228, 52), (128, 444, 7)]
+
+
+@pytest.mark.parametrize("n", SPLIT_SIZES)
 @pytest.mark.parametrize("flavour", FLAVOURS)
 def test_every_plane_of_every_column_once(flavour, n):
     """A step through each tile configuration (each splits the mesh differently)

@@ -9,6 +9,7 @@ import textwrap
 import pytest
 
 from astaroth_b200 import abi
+from test_gpu_partition import SPLIT_SIZES
 
 TESTS = os.path.dirname(os.path.abspath(__file__))
 FLAVOURS = ("sp", "dp", "mixed")
@@ -165,3 +166,36 @@ def test_a_mesh_that_is_not_all_mapped_is_refused(fake_runtime, tmp_path, flavou
         rc, launches = load_and_store(dev, mesh(base))
         assert rc == (1, 1) and launches > 2
     """)
+
+
+@pytest.mark.parametrize("flavour", FLAVOURS)
+def test_the_split_takes_every_form(fake_runtime, tmp_path, flavour):
+    """The sizes at which test_gpu_partition.py compares the split of the columns
+    reach, between them and the tile configurations, every form that it can take."""
+    run(fake_runtime, tmp_path, flavour, f"sizes = {SPLIT_SIZES}\n" + """
+from astaroth_b200 import Device
+forms = set()
+for n in sizes:
+    dev = Device(flavour, abi.make_info(prec, *n))
+    for cfg in range(dev.solve_config()[1]):
+        dev.set_solve_config(cfg)
+        dev.integrate_substep(0, 1e-3)
+        w = (ctypes.c_int * 30)()
+        fake.fake_last_solve(w)
+        assert tuple(w[3:6]) == n and w[21] == n[2]  # Layout::nx, ny, nz; SolveGeom::nzr
+        nfull, rem0, rem, slabs, slab_planes, left, zseg, seg_tasks = w[22:30]
+        if seg_tasks:
+            forms.add("segments")
+            continue
+        if nfull:
+            forms.add("whole, then slabs" if rem else "whole")
+        elif slabs > 1:
+            forms.add("slabs")
+        if left:
+            forms.add("shares")
+            if rem > 148 - slabs * rem:
+                forms.add("shares across columns")
+    dev.destroy()
+want = {"segments", "whole, then slabs", "whole", "slabs", "shares", "shares across columns"}
+assert forms == want, want - forms
+""")
