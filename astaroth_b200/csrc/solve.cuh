@@ -580,9 +580,11 @@ rhs_from(const PT& P, const Terms<T>& m, T roc[ACB_NF])
     const T inv_rho = rexp<T>(-m.lnrho);
     const T inv_T   = rrcp<T>(P.exp_lnT0 * expE);
 
-    // continuity: -u.grad(lnrho) - div(u)
+    // continuity: -u.grad(lnrho) - div(u), the products summed first: added one
+    // by one to the divergence, as a rule the larger term, they would round it
+    // three times (mixed 512^3, 53 steps: lnrho 2.7e-7 off instead of 2.2e-7)
     const T divu = m.g[0][0] + m.g[1][1] + m.g[2][2];
-    roc[0] = -rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], rfma(m.u[2], m.glr[2], divu)));
+    roc[0] = -(rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], m.u[2] * m.glr[2])) + divu);
 
     // induction: u x B + eta lap(A)
     roc[4] = rfma(m.u[1], m.b[2], rfma(-m.u[2], m.b[1], m.resist[0]));
@@ -631,10 +633,8 @@ rhs_from(const PT& P, const Terms<T>& m, T roc[ACB_NF])
         const T q = rfma(P.gamma, pr[i], -m.glr[i]);
         cond      = rfma(q, q, cond);
     }
-    T r    = rfma(inv_T, heat, (P.k_heat * inv_rho) * cond);
-    r      = rfma(-m.u[0], m.gs[0], r);
-    r      = rfma(-m.u[1], m.gs[1], r);
-    roc[7] = rfma(-m.u[2], m.gs[2], r);
+    const T adv = rfma(m.u[0], m.gs[0], rfma(m.u[1], m.gs[1], m.u[2] * m.gs[2]));
+    roc[7]      = rfma(inv_T, heat, (P.k_heat * inv_rho) * cond) - adv;
 }
 
 // Register queues of one thread's column along z: the values of each array at
