@@ -331,24 +331,29 @@ acb_host::make_params(const AcMeshInfo& uniforms, const Layout& L, int step, int
     const double gamma = rp[AC_gamma], cp = rp[AC_cp_sound], mu0 = rp[AC_mu0];
     const double nu = rp[AC_nu_visc], eta = rp[AC_eta], zeta = rp[AC_zeta];
     const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2}; // xy, xz, yz
+    // 3/2 / ds^2 of the finest axis without its power of two (RhsParams::inv_mu0)
+    const double finest = std::max({fabs(inv[0]), fabs(inv[1]), fabs(inv[2])});
+    const double unit   = 3.0 / 2.0 * finest * finest;
+    int exponent;
+    const double j_unit = unit > 0.0 && isfinite(unit) ? 2.0 * frexp(unit, &exponent) : 1.0;
     for (int a = 0; a < 3; ++a) {
         const double s2 = 3.0 / 2.0 * inv[a] * inv[a];
         const double cx = 3.0 / 8.0 * inv[pa[a]] * inv[pb[a]];
         R.s1[a]         = (AcReal)(3.0 / 4.0 * inv[a]);
-        R.s2[a]         = (AcReal)s2;
+        R.s2[a]         = (AcReal)(s2 / j_unit);
         R.perp_u[a]     = (AcReal)(s2 * nu);
         R.own_u[a]      = (AcReal)(s2 * (4.0 / 3.0 * nu + zeta));
         R.eta_a[a]      = (AcReal)(s2 * eta);
         R.cond_s[a]     = (AcReal)(s2 * (gamma / cp));
         R.cond_l[a]     = (AcReal)(s2 * (gamma - 1.0));
         R.cross_u[a]    = (AcReal)(cx * (nu / 3.0 + zeta));
-        R.cross_a[a]    = (AcReal)cx;
+        R.cross_a[a]    = (AcReal)(cx / j_unit);
     }
     R.nu          = rp[AC_nu_visc];
     R.two_nu      = (AcReal)(2.0 * nu);
     R.zeta        = rp[AC_zeta];
-    R.inv_mu0     = (AcReal)(1.0 / mu0);
-    R.k_ohm       = (AcReal)(eta * mu0 / (mu0 * mu0));
+    R.inv_mu0     = (AcReal)(j_unit / mu0);
+    R.k_ohm       = (AcReal)(eta * mu0 / (mu0 * mu0) * j_unit * j_unit);
     R.gamma_cp    = (AcReal)(gamma / cp);
     R.inv_cp      = (AcReal)(1.0 / cp);
     R.gamma       = (AcReal)gamma;

@@ -69,3 +69,50 @@ def test_continuity_rounds_the_divergence_once():
     print(f"continuity: rms error {got:.3e}, in this order {want:.3e}")
     # 2.6e5 vertices: the rms of either is known to 0.3 %
     assert got <= 1.02 * want
+
+
+def test_ohmic_heating_has_no_factor():
+    """With u = lnrho = s = 0 the entropy's rate is eta mu0 j^2 / (rho T), j of second
+    derivatives. It is off by one factor where their scale 3/2 / ds^2 is rounded, at
+    a spacing where that rounding is nearly as large as it gets. What remains
+    is the rounding of one product of parameters and that of the stencil's
+    coefficients: -1/10 and 1/135 as floats leave a smooth derivative off by 1.1e-8."""
+    inv = np.float32(13.0)
+    off = lambda v: float(np.float32(1.5 * float(v) ** 2)) / (1.5 * float(v) ** 2) - 1  # noqa: E731
+    while abs(off(inv)) < 5.5e-8:
+        inv = np.nextafter(inv, np.float32(14.0))
+    inv = float(inv)
+    rng = np.random.default_rng(3)
+    fields = [np.zeros((N + 2 * G,) * 3) for _ in range(8)]
+    for w in (abi.VTXBUF_AX, abi.VTXBUF_AY, abi.VTXBUF_AZ):
+        a = rng.uniform(-1e-3, 1e-3, (N,) * 3).astype(np.float32).astype(np.float64)
+        fields[w] = np.pad(a, G, mode="wrap")
+    eta, mu0 = 2.0 ** -8, 1.0
+    got = rate(fields, abi.VTXBUF_ENTROPY, inv, eta=eta, mu0=mu0, lnT0=0.0, lnrho0=0.0,
+               gamma=5 / 3, nu_visc=5e-3, cs_sound=1.0, cp_sound=1.0)
+    A = fields[abi.VTXBUF_AX:abi.VTXBUF_AZ + 1]
+    pure = [[sum(c * (shifted(A[i], a, k) + shifted(A[i], a, -k) - 2 * shifted(A[i], a, 0))
+                 for k, c in ((1, 1.5), (2, -0.15), (3, 1 / 90))) for a in range(3)]
+            for i in range(3)]
+
+    def cross(f, a, b):
+        out = 0
+        for k, c in ((1, 270 / 720), (2, -27 / 720), (3, 2 / 720)):
+            for sa, sb in ((1, 1), (-1, -1), (1, -1), (-1, 1)):
+                s = [0, 0, 0]
+                s[2 - a], s[2 - b] = sa * k, sb * k
+                out = out + c * sa * sb * f[tuple(slice(G + d, G + N + d) for d in s)]
+        return out
+
+    j2 = 0
+    for i in range(3):
+        j = sum(cross(A[k], min(i, k), max(i, k)) for k in range(3) if k != i)
+        j2 = j2 + (j - sum(pure[i][a] for a in range(3) if a != i)) ** 2
+    want = eta * mu0 * j2 * (inv * inv / mu0) ** 2
+    factor = float(((got - want) * want).sum() / (want * want).sum())
+    unit = 2.0 * math.frexp(1.5 * inv * inv)[0]
+    k = eta / mu0 * unit * unit
+    bound = abs(float(np.float32(k)) / k - 1) + 2 * 1.1e-8
+    print(f"heating: off by {factor:.2e}, bound {bound:.2e}, the scale alone {2 * off(inv):.2e}")
+    assert bound < 0.5 * abs(2 * off(inv))
+    assert abs(factor) <= bound
