@@ -410,12 +410,16 @@ acb_host::make_params(const AcMeshInfo& uniforms, const Layout& L, int step, int
 // fill its ring and prime its queues before its first output. The split is the
 // one with the smallest score, the time of the longest CTA plus the average over
 // the SMs: the former is what a mesh alone waits for, the latter what several in
-// flight share. Two forms compete:
-//   - whole columns, and the rem < slots columns of the last wave cut into slabs;
-//     what the slabs leave is shared by the CTAs that have none (at staggered z,
-//     where neighbours share fewer halos in L2: 4 % dearer, and 1 % for what runs
-//     beside it, the mixed build's 192^3 and 512^3 steps as measured);
+// flight share. Three forms compete:
+//   - whole columns, and the rem < slots columns of the last wave cut into slabs,
+//     one for a CTA;
+//   - the same with shorter slabs, what they leave shared by the CTAs that have none
+//     (at staggered z, where neighbours share fewer halos in L2: 4 % dearer, and 1 %
+//     for what runs beside it, the mixed build's 192^3 and 512^3 steps as measured);
 //   - uniform z segments, dealt in several rounds.
+// A lone mesh is what the weights serve: several in flight can take longer than with
+// fewer, longer pieces (10 FP64 steps of 61 x 70 x 53 with three Devices in flight
+// 925 us instead of 693 without this split; alone 1063 instead of 1784).
 // Against uniform segments of at least 16 planes alone, a step of a 32^3 FP32 mesh
 // takes 29 us instead of 102, 64^3 57 instead of 107, 112^3 200 instead of 205 (FP64
 // 39, 91 and 352 instead of 139, 147 and 382).
@@ -477,11 +481,6 @@ split_columns(SolveGeom& g, int slots, double piece_cost, double* score)
         return slots;
     return g.slabs * g.rem;
 }
-
-// Time of starting a piece, in planes of the first configuration's tile (FP32: a
-// substep takes about 6 us, launch included, and 1.65 us per plane of its longest
-// CTA).
-constexpr double kPieceCost = 3.0;
 
 // The tiles of a launch over the box [s, e) and their split over the CTAs.
 static int

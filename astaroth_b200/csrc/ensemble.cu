@@ -142,23 +142,22 @@ drop_graphs(Ensemble e)
 // launch over `slots` CTAs. Full rounds of units are dealt round-robin, so that
 // the CTAs of a round stream neighbouring tiles at the same z and share their
 // halos in L2. With `level`, the units of the last, partial round are cut so
-// that all CTAs end together, counting kPieceCost planes for each piece (the
+// that all CTAs end together, counting piece_cost planes for each piece (the
 // time to fill its ring and prime its queues): the CTAs take the units' first
 // planes in step, as many units as there are CTAs at a time, and the CTAs left
 // over share what remains of the units, running from one to the next. Without
 // it they go to one CTA each. (64 FP32 meshes of 32^3 ... 128^3: 0.7 % of a step
 // against z segments of 32 planes dealt round-robin.)
 void
-schedule(const std::vector<Piece>& units, int slots, bool level,
+schedule(const std::vector<Piece>& units, int slots, int piece_cost, bool level,
          std::vector<std::vector<Piece>>& cta)
 {
-    constexpr int kPieceCost = 2;
     cta.assign(slots, {});
     std::vector<int> load(slots, 0);
     const int n = (int)units.size(), full = n / slots * slots, rem = n - full;
     for (int i = 0; i < (level ? full : n); ++i) {
         cta[i % slots].push_back(units[i]);
-        load[i % slots] += units[i].n + kPieceCost;
+        load[i % slots] += units[i].n + piece_cost;
     }
     if (!level || rem == 0)
         return;
@@ -168,7 +167,7 @@ schedule(const std::vector<Piece>& units, int slots, bool level,
     for (int i = full; i < n; ++i)
         sum += units[i].n;
     std::vector<std::vector<Piece>> tail;
-    for (long long T = (sum + slots - 1) / slots + kPieceCost;; T += std::max(1LL, T / 256)) {
+    for (long long T = (sum + slots - 1) / slots + piece_cost;; T += std::max(1LL, T / 256)) {
         tail.assign(slots, {});
         std::vector<Piece> left(units.begin() + full, units.end());
         auto take = [&](int c, Piece& u, long long room) {
@@ -184,11 +183,11 @@ schedule(const std::vector<Piece>& units, int slots, bool level,
         };
         const int in_step = slots / rem * rem;
         for (int c = 0; c < in_step; ++c)
-            take(c, left[c % rem], T - load[c] - kPieceCost);
+            take(c, left[c % rem], T - load[c] - piece_cost);
         int i = 0;
         for (int c = in_step; c < slots; ++c)
-            for (long long room = T - load[c] - kPieceCost; room > 0 && i < rem;) {
-                room -= take(c, left[i], room) + kPieceCost;
+            for (long long room = T - load[c] - piece_cost; room > 0 && i < rem;) {
+                room -= take(c, left[i], room) + piece_cost;
                 if (left[i].n == 0)
                     ++i;
             }
@@ -219,6 +218,7 @@ build_tables(Ensemble e, int config, int seg_planes)
     ACB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg.kern[1], cfg.threads,
                                                                  cfg.smem));
     per_sm = std::max(per_sm, 1);
+    const int piece_cost = (int)lround(kPieceCost / cfg.plane_cost);
     // planes per unit of a member: its z range in equal segments
     auto zseg_of = [&](const Layout& L) {
         int nseg = 1;
@@ -286,7 +286,7 @@ build_tables(Ensemble e, int config, int seg_planes)
                     units.push_back(Piece{t, z0, std::min(zseg, g.nzr - z0), pos - g0});
         }
         std::vector<std::vector<Piece>> cta;
-        schedule(units, e->num_sms * per_sm, seg_planes == 0, cta);
+        schedule(units, e->num_sms * per_sm, piece_cost, seg_planes == 0, cta);
         piece_at.push_back(pieces.size());
         first_at.push_back(first.size());
         int grid = 0, at = 0;
@@ -423,7 +423,7 @@ enqueue_step(Ensemble e, cudaStream_t st, AcReal dt)
 // What a cached choice was timed for: the GPU, the compiled tiles that its index
 // counts, how segment lengths are dealt (raised when schedule() changes), and
 // the members. One word: the cache file separates by blanks.
-constexpr int kScheduleVersion = 2;
+constexpr int kScheduleVersion = 3;
 
 std::string
 cache_key(Ensemble e)

@@ -45,6 +45,11 @@ constexpr double kPlaneCost[3] = {1.0, 0.715, 0.73};
 constexpr double kPlaneCost[3] = {1.0, 0.70, 1.05};
 #endif
 
+// Time of starting a piece, in planes of the first configuration's tile (FP32: a
+// substep takes about 6 us, launch included, and 1.65 us per plane of its longest
+// CTA). 4 steps of 64 FP32 meshes of 32^3 ... 128^3 take 24.35 ms, counting 2 24.59.
+constexpr double kPieceCost = 3.0;
+
 typedef void (*SolveKernelFn)(const CUtensorMap, const SolveArgs<AcReal>, const CentreMaps);
 typedef void (*EnsKernelFn)(const CUtensorMap, const EnsSolveArgs<AcReal>, const CentreMaps);
 
@@ -185,7 +190,8 @@ void stage_destroy(StageBuf* stage);
 
 // copies a flat range of a field (field: its base, block + fidx(L, f, 0))
 // between the caller's memory (reference order) and the padded device layout,
-// through the staging buffer unless it is this GPU's memory; zeroes the lo parts of loaded values when given.
+// through the staging buffer unless it is this GPU's memory; zeroes the lo parts
+// of loaded values when given.
 AcResult copy_field_range(cudaStream_t st, const Layout& L, state_t* field, size_t s,
                           AcReal* host, size_t count, bool h2d, lo16_t* lo_field,
                           StageBuf* stage);

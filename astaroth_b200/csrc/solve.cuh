@@ -394,8 +394,8 @@ sum3(V c2, V c3, const V* d)
 // - f0: for a smooth field u and v are exact in FP32 (Sterbenz), so f(+k) + f(-k)
 // - 2 f0 keeps its digits instead of cancelling terms of size |c0 f0| (about
 // 2.7 f / ds^2); mathematically the same stencil (c0 = -2 (c1 + c2 + c3)). This
-// is what brings the mixed build within 2.2e-7 of FP64. It is evaluated as S =
-// 2 (f(-k) - f0) + (f(+k) - f(-k)), one fused multiply-add on the two exact
+// is what brings the mixed build from 2.3e-6 to 2.2e-7 of FP64. It is evaluated as
+// S = 2 (f(-k) - f0) + (f(+k) - f(-k)), one fused multiply-add on the two exact
 // differences (the first difference is formed anyway). The other builds, whose
 // error is that of their state, take the plain sums f(+k) + f(-k) and add c0 f0
 // (two operations per point pair instead of three).
@@ -1506,8 +1506,7 @@ consume_task(const SolveArgs<AcReal>& a, const SolveGeom& gv, const PT& P,
             }
         }
         __syncwarp();
-        // with the queues the centre plane is done with; without them the
-        // plane three below it
+        // the centre plane is done with: what later planes need of it is queued
         if (lane == 0)
             mbar_arrive(&empty[(q + p + NGHOST) % NP]);
         if constexpr (CT) {
