@@ -340,10 +340,12 @@ acb_host::make_params(const AcMeshInfo& uniforms, const Layout& L, int step, int
         const double s2 = 3.0 / 2.0 * inv[a] * inv[a];
         const double cx = 3.0 / 8.0 * inv[pa[a]] * inv[pb[a]];
         R.s1[a]         = (AcReal)(3.0 / 4.0 * inv[a]);
+#if ACB_MIXED
         // (1/45 itself where s1 has no such rounding: no spacing, or one at the
         // type's limits)
         const double r3 = (inv[a] / R.s1[a] - 2.0 + 4.0 * (double)(AcReal)(1.0 / 5.0)) / 6.0;
         R.r3[a]         = (AcReal)(fabs(r3 - 1.0 / 45.0) < 1e-7 ? r3 : 1.0 / 45.0);
+#endif
         R.s2[a]         = (AcReal)(s2 / j_unit);
         R.perp_u[a]     = (AcReal)(s2 * nu);
         R.own_u[a]      = (AcReal)(s2 * (4.0 / 3.0 * nu + zeta));

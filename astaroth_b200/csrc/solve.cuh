@@ -55,7 +55,6 @@
 template <typename T>
 struct RhsParams {
     T s1[3];                  // first derivative: axis; 3/4 / ds
-    T r3[3];                  // its last coefficient: axis (StencilCoefs; mixed build)
     T s2[3];                  // second derivative: axis; 3/2 / ds^2, over j_unit
     T perp_u[3], own_u[3];    // s2 times nu (across the component's axis), and times
                               // 4/3 nu + zeta (along it)
@@ -74,6 +73,9 @@ struct RhsParams {
     T gamma_cp; // gamma / cp
     T inv_cp, gamma, gm1, lnrho0, cs2_sound, k_heat;
     T exp_lnT0; // exp(lnT0): T = exp(lnT0 + E) = exp_lnT0 * exp(E)
+#if ACB_MIXED
+    T r3[3]; // first derivative's last coefficient: axis (StencilCoefs)
+#endif
 };
 
 template <typename T>
@@ -117,7 +119,7 @@ struct __align__(16) Piece {
 };
 
 // One member of an ensemble (many independent meshes advanced by one launch):
-// the TMA map of its `in` block, its geometry and task range and its buffers.
+// the TMA map of its `in` block, its geometry and its buffers.
 // Kept in global memory, one table per buffer parity; its parameters travel
 // with the launch (EnsSolveArgs::mp).
 template <typename T>
@@ -192,10 +194,11 @@ struct TileCfg {
     static constexpr int CONSUMERS = TX_ * TY_;        // one thread per (x, y) column
     static constexpr int CWARPS    = CONSUMERS / 32;   // consumer warps
     // With 8 or 12 consumer warps the producer is a whole warpgroup (4 warps,
-    // one of them working) that hands its registers to the consumers (setmaxnreg), so each consumer thread gets the registers its z
-    // queues need. An SM sub-partition's 16K registers hold 2 consumer warps
-    // and 1 producer warp (2 * 232 + 40 = 504 <= 512 registers a lane), or 3
-    // and 1 (3 * 160 + 32 = 512): more warps to hide latency, fewer registers.
+    // one of them working) that hands its registers to the consumers
+    // (setmaxnreg), so each consumer thread gets the registers its z queues
+    // need. An SM sub-partition's 16K registers hold 2 consumer warps and 1
+    // producer warp (2 * 232 + 40 = 504 <= 512 registers a lane), or 3 and 1
+    // (3 * 160 + 32 = 512): more warps to hide latency, fewer registers.
     static constexpr bool WGSPEC = CWARPS == 8 || CWARPS == 12;
     static constexpr int THREADS = CONSUMERS + (WGSPEC ? 128 : 32); // plus the producer
     static constexpr int REG_CONSUMER = CWARPS == 12 ? 160 : 232;
@@ -607,11 +610,16 @@ rhs_from(const PT& P, const Terms<T>& m, T roc[ACB_NF])
     const T inv_rho = rexp<T>(-m.lnrho);
     const T inv_T   = rrcp<T>(P.exp_lnT0 * expE);
 
-    // continuity: -u.grad(lnrho) - div(u), the products summed first: added one
-    // by one to the divergence, as a rule the larger term, they would round it
-    // three times (mixed 512^3, 53 steps: lnrho 2.7e-7 off instead of 2.2e-7)
+    // continuity: -u.grad(lnrho) - div(u). The mixed build sums the products first:
+    // added one by one to the divergence, as a rule the larger term, they would
+    // round it three times (512^3, 53 steps: lnrho 2.7e-7 off FP64 instead of
+    // 2.2e-7). The FP32 build's error is its state's either way, and it is about 1 %
+    // faster with one operation less.
     const T divu = m.g[0][0] + m.g[1][1] + m.g[2][2];
-    roc[0] = -(rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], m.u[2] * m.glr[2])) + divu);
+    if constexpr (ACB_MIXED)
+        roc[0] = -(rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], m.u[2] * m.glr[2])) + divu);
+    else
+        roc[0] = -rfma(m.u[0], m.glr[0], rfma(m.u[1], m.glr[1], rfma(m.u[2], m.glr[2], divu)));
 
     // induction: u x B + eta lap(A)
     roc[4] = rfma(m.u[1], m.b[2], rfma(-m.u[2], m.b[1], m.resist[0]));
@@ -660,8 +668,10 @@ rhs_from(const PT& P, const Terms<T>& m, T roc[ACB_NF])
         const T q = rfma(P.gamma, pr[i], -m.glr[i]);
         cond      = rfma(q, q, cond);
     }
-    const T adv = rfma(m.u[0], m.gs[0], rfma(m.u[1], m.gs[1], m.u[2] * m.gs[2]));
-    roc[7]      = rfma(inv_T, heat, (P.k_heat * inv_rho) * cond) - adv;
+    T r    = rfma(inv_T, heat, (P.k_heat * inv_rho) * cond);
+    r      = rfma(-m.u[0], m.gs[0], r);
+    r      = rfma(-m.u[1], m.gs[1], r);
+    roc[7] = rfma(-m.u[2], m.gs[2], r);
 }
 
 // Register queues of one thread's column along z: the values of each array at
@@ -1661,7 +1671,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     grid_wait();
 
     if constexpr (Cfg::WGSPEC) {
-        // whole warpgroups: warps 0..7 consume, warps 8..11 produce
+        // whole warpgroups: the first two or three consume, the last produces
         if (warp >= CWARPS)
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Cfg::REG_PRODUCER));
         else
