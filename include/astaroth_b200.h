@@ -175,7 +175,8 @@ AcResult acEnsembleGetStatus(Ensemble ensemble, unsigned* status);
 AcResult acEnsembleGetCudaStream(Ensemble ensemble, void** cuda_stream);
 AcResult acEnsembleGetLaunchCount(Ensemble ensemble, unsigned long long* count);
 /* Schedule: tile configuration (index into the compiled table) and the target
- * number of planes per z segment of a task (0 = whole columns). */
+ * number of planes per z segment of a task (0 = whole columns, as in a new
+ * ensemble). A schedule that is refused leaves the one in use. */
 AcResult acEnsembleSetSchedule(Ensemble ensemble, const int config, const int segment_planes);
 AcResult acEnsembleGetSchedule(Ensemble ensemble, int* config, int* segment_planes);
 /* Times every (configuration, segment length) pair on this ensemble and keeps
